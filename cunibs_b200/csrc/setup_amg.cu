@@ -581,11 +581,19 @@ __global__ void compose_kernel(int* __restrict__ agg, const int* __restrict__ st
 // the lower triangle of the matrix padded to a multiple of kSweepB with an identity block. Sweeping
 // pivot block k with P = A_kk^-1 maps
 //   A_kk -> -P,  A_ik -> C_i = A_ik P,  A_ij -> A_ij - C_i A_kj   (i, j != k),
-// and after every block has been swept the matrix holds -A^-1. Only tiles on or below the block
-// diagonal are stored and updated (A_kj for j > k is read as A_jk^T), so a step is one SYRK-shaped
-// product of about n^2 kSweepB multiply-adds; the whole inverse costs n^3 of them, on every SM.
+// and after every block has been swept the matrix holds -A^-1. Only blocks on or below the block
+// diagonal hold values that are used (A_kj for j > k is read as A_jk^T), so a step is one SYRK-shaped
+// product of about n^2 kSweepB / 2 multiply-adds; the whole inverse costs n^3 / 2 of them.
+// Two launches a step: sweep_panel_kernel (the swept row and column of the pivot block, and the
+// product's two operands), then sweep_update_kernel, whose first block also inverts the next pivot
+// block, which depends on its own tile alone: a serial chain of 64 pivots that would otherwise leave the
+// GPU idle between two steps.
+// Measured on the 6,763 rows of a 0.68M-tet head's level 1: with the pivot block inverted by a launch of its
+// own (0.21 ms of one block) and 64 x 64 update tiles of 4 x 4 patches staged in two halves (0.25 ms a step),
+// 56 ms; set-up to the first result 89-95 ms, 54 ms with this form.
 
 constexpr int kSweepB = 64;
+constexpr int kSweepRows = 128;  // rows of an update tile (two blocks), by kSweepB columns
 
 __global__ void densify_lower_kernel(const int* __restrict__ ptr, const int* __restrict__ col,
                                      const double* __restrict__ val, int n, int N, double* __restrict__ m) {
@@ -598,166 +606,229 @@ __global__ void densify_lower_kernel(const int* __restrict__ ptr, const int* __r
     for (int p = ptr[i]; p < ptr[i + 1]; ++p) m[static_cast<long>(i) * N + col[p]] = val[p];
 }
 
-// Tile (I, J) of the symmetric matrix as stored (lower triangle): element (r, c) of the tile.
-__device__ __forceinline__ double sym_tile(const double* __restrict__ m, int N, int I, int J, int r, int c) {
-    const long row = static_cast<long>(I) * kSweepB + r, col = static_cast<long>(J) * kSweepB + c;
-    return (I > J || (I == J && r >= c)) ? m[row * N + col] : m[col * N + row];
+// pinv = A^-1 of the 64 x 64 SPD block whose lower triangle sits in `tile` (rows of kSweepB + 1), by a scalar
+// sweep of its 64 pivots (which leaves -A^-1). Each of 256 threads keeps a 4 x 4 patch in registers; a
+// pivot's row goes through shared memory (one barrier a pivot, two buffers), and serves as its column
+// too: the update a_ij - (a_ip a_pj) / d keeps the block symmetric to the last bit. status = 1 when a pivot is
+// not positive (not SPD).
+__device__ void invert_block(const double* tile, double (*row)[kSweepB], double* __restrict__ pinv,
+                             int* __restrict__ status) {
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+    double v[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int i = ty * 4 + a, j = tx * 4 + b;
+            v[a][b] = i >= j ? tile[i * (kSweepB + 1) + j] : tile[j * (kSweepB + 1) + i];
+        }
+    for (int q = 0; q < kSweepB / 4; ++q) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {  // pivot 4 q + u: row u of the threads with ty = q
+            double* rb = row[u & 1];
+            if (ty == q) {
+#pragma unroll
+                for (int b = 0; b < 4; ++b) rb[tx * 4 + b] = v[u][b];
+            }
+            __syncthreads();
+            double d = rb[4 * q + u];
+            if (!(d > 0.0)) {
+                if (threadIdx.x == 0) *status = 1;
+                d = 1.0;
+            }
+            const double inv = 1.0 / d;
+            double ri[4], rj[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                ri[a] = rb[ty * 4 + a];
+                rj[a] = rb[tx * 4 + a];
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const bool pi = ty == q && a == u, pj = tx == q && b == u;
+                    const double upd = v[a][b] - (ri[a] * rj[b]) * inv;
+                    v[a][b] = pi && pj ? -inv : (pi ? rj[b] * inv : (pj ? ri[a] * inv : upd));
+                }
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) pinv[(ty * 4 + a) * kSweepB + tx * 4 + b] = -v[a][b];
 }
 
-// acc (per thread a 4 x 4 patch of a 64 x 64 tile) = X (64 x 64, rows ldx apart) * Y (64 x 64, rows
-// ldy apart); the reduction dimension in chunks of 32 staged (coalesced loads) in `stage`, a
-// shared-memory buffer of kStageDoubles.
-constexpr int kStageDoubles = kSweepB * 33 + 32 * kSweepB;
+// pinv of pivot block 0 (the others are inverted by sweep_update_kernel).
+__global__ void __launch_bounds__(256) sweep_pivot_kernel(const double* __restrict__ m, int N,
+                                                          double* __restrict__ pinv, int* __restrict__ status) {
+    __shared__ double tile[kSweepB * (kSweepB + 1)];
+    __shared__ double row[2][kSweepB];
+    for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x)
+        tile[q / kSweepB * (kSweepB + 1) + q % kSweepB] = m[static_cast<long>(q / kSweepB) * N + q % kSweepB];
+    __syncthreads();
+    invert_block(tile, row, pinv, status);
+}
 
-__device__ __forceinline__ void tile_product(const double* X, long ldx, const double* Y, long ldy, double acc[4][4],
-                                             double* stage) {
-    double (*xs)[33] = reinterpret_cast<double (*)[33]>(stage);
-    double (*ys)[kSweepB] = reinterpret_cast<double (*)[kSweepB]>(stage + kSweepB * 33);
-    const int t = threadIdx.x, ty = t / 16, tx = t % 16;
+// For every block row I != k (blockIdx.x = I): the old row panel rbuf[:, I] = A_kI and C_I^T = P A_kI in
+// cbuf[:, I] (both 64 x N; P is symmetric), and the swept A_Ik = C_I (A_kI = C_I^T above the diagonal) in
+// their place; A_kk = -P.
+__global__ void __launch_bounds__(256) sweep_panel_kernel(double* __restrict__ m, int N, int k,
+                                                          const double* __restrict__ pinv, double* __restrict__ cbuf,
+                                                          double* __restrict__ rbuf) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    double* ps = reinterpret_cast<double*>(sweep_smem);  // P, 64 x 64
+    double* as = ps + kSweepB * kSweepB;                 // A_kI, rows of kSweepB + 2
+    constexpr int LD = kSweepB + 2;
+    const int I = blockIdx.x;
+    const long at_kI = static_cast<long>(k) * kSweepB * N + static_cast<long>(I) * kSweepB;
+    const long at_Ik = static_cast<long>(I) * kSweepB * N + static_cast<long>(k) * kSweepB;
+    if (I == k) {
+        for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x)
+            m[at_kI + static_cast<long>(q / kSweepB) * N + q % kSweepB] = -pinv[q];
+        return;
+    }
+    for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x) {
+        const int r = q / kSweepB, c = q % kSweepB;
+        ps[q] = pinv[q];
+        // Read along the stored rows: A_kI itself above the diagonal block, A_Ik below it.
+        if (I < k) as[r * LD + c] = m[at_kI + static_cast<long>(r) * N + c];
+        else as[c * LD + r] = m[at_Ik + static_cast<long>(r) * N + c];
+    }
+    __syncthreads();
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+    double acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    for (int k0 = 0; k0 < kSweepB; k0 += 32) {
-        for (int q = t; q < kSweepB * 32; q += blockDim.x) {
-            xs[q / 32][q % 32] = X[(q / 32) * ldx + k0 + q % 32];
-            ys[q / kSweepB][q % kSweepB] = Y[(k0 + q / kSweepB) * ldy + q % kSweepB];
-        }
-        __syncthreads();
 #pragma unroll 8
-        for (int kk = 0; kk < 32; ++kk) {
-            double xa[4];
+    for (int kk = 0; kk < kSweepB; ++kk) {
+        double xa[4];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) xa[a] = xs[ty * 4 + a][kk];
-            const double2 y0 = *reinterpret_cast<const double2*>(&ys[kk][tx * 4]);
-            const double2 y1 = *reinterpret_cast<const double2*>(&ys[kk][tx * 4 + 2]);
-            const double yb[4] = {y0.x, y0.y, y1.x, y1.y};
+        for (int a = 0; a < 4; ++a) xa[a] = ps[kk * kSweepB + ty * 4 + a];  // P is symmetric
+        const double2 y0 = *reinterpret_cast<const double2*>(as + kk * LD + tx * 4);
+        const double2 y1 = *reinterpret_cast<const double2*>(as + kk * LD + tx * 4 + 2);
+        const double yb[4] = {y0.x, y0.y, y1.x, y1.y};
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) acc[a][b] = fma(xa[a], yb[b], acc[a][b]);
-        }
-        __syncthreads();
+            for (int b = 0; b < 4; ++b) acc[a][b] = fma(xa[a], yb[b], acc[a][b]);
     }
-}
-
-// P = A_kk^-1 of the current pivot block, by a scalar sweep of its 64 pivots in shared memory
-// (which leaves -A_kk^-1). status = 1 when a pivot is not positive (not SPD).
-__global__ void __launch_bounds__(256) sweep_pivot_kernel(const double* __restrict__ m, int N, int k,
-                                                          double* __restrict__ pinv, int* __restrict__ status) {
-    __shared__ double b[kSweepB][kSweepB + 1];
-    __shared__ double dsh;
-    for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x)
-        b[q / kSweepB][q % kSweepB] = sym_tile(m, N, k, k, q / kSweepB, q % kSweepB);
-    __syncthreads();
-    for (int p = 0; p < kSweepB; ++p) {
-        if (threadIdx.x == 0) {
-            double d = b[p][p];
-            if (!(d > 0.0)) {
-                *status = 1;
-                d = 1.0;
-            }
-            dsh = d;
-        }
-        __syncthreads();
-        const double d = dsh;
-        for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x) {
-            const int i = q / kSweepB, j = q % kSweepB;
-            if (i != p && j != p) b[i][j] -= b[i][p] * b[p][j] / d;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < kSweepB; i += blockDim.x) {
-            if (i != p) {
-                b[i][p] /= d;
-                b[p][i] /= d;
-            }
-        }
-        if (threadIdx.x == 0) b[p][p] = -1.0 / d;
-        __syncthreads();
-    }
-    // P is symmetric; its two rounded halves are averaged so that it is so exactly.
-    for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x) {
-        const int i = q / kSweepB, j = q % kSweepB;
-        pinv[q] = -0.5 * (b[i][j] + b[j][i]);
-    }
-}
-
-// For every block row I != k (blockIdx.x = I): the old row panel rbuf[:, I] = A_kI (64 x N, rows N
-// apart) and C_I = A_Ik P into cbuf (N x 64), formed as C_I^T = P A_kI (P is symmetric).
-__global__ void __launch_bounds__(256) sweep_panel_kernel(const double* __restrict__ m, int N, int k,
-                                                          const double* __restrict__ pinv, double* __restrict__ cbuf,
-                                                          double* __restrict__ rbuf) {
-    __shared__ __align__(16) double buf[kStageDoubles];
-    static_assert(kStageDoubles >= kSweepB * (kSweepB + 1), "the staging buffer holds one padded tile");
-    double (*tile)[kSweepB + 1] = reinterpret_cast<double (*)[kSweepB + 1]>(buf);  // A_kI
-    const int I = blockIdx.x;
-    if (I == k) return;
-    for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x) {
-        // Read along the stored rows: A_kI itself above the diagonal block, A_Ik below it.
-        if (I < k) {
-            const int r = q / kSweepB, c = q % kSweepB;
-            tile[r][c] = m[(static_cast<long>(k) * kSweepB + r) * N + static_cast<long>(I) * kSweepB + c];
-        } else {
-            const int c = q / kSweepB, r = q % kSweepB;
-            tile[r][c] = m[(static_cast<long>(I) * kSweepB + c) * N + static_cast<long>(k) * kSweepB + r];
-        }
-    }
-    __syncthreads();
     for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x) {
         const int r = q / kSweepB, c = q % kSweepB;
-        rbuf[static_cast<long>(r) * N + static_cast<long>(I) * kSweepB + c] = tile[r][c];
+        rbuf[static_cast<long>(r) * N + static_cast<long>(I) * kSweepB + c] = as[r * LD + c];
     }
     __syncthreads();
-    double acc[4][4];
-    tile_product(pinv, kSweepB, rbuf + static_cast<long>(I) * kSweepB, N, acc, buf);
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
-            cbuf[(static_cast<long>(I) * kSweepB + tx * 4 + b) * kSweepB + ty * 4 + a] = acc[a][b];
-}
-
-// A_IJ -= C_I A_kJ for the stored tiles I >= J with I, J != k (blockIdx = (J, I)).
-__global__ void __launch_bounds__(256) sweep_update_kernel(double* __restrict__ m, int N, int k,
-                                                           const double* __restrict__ cbuf,
-                                                           const double* __restrict__ rbuf) {
-    __shared__ __align__(16) double buf[kStageDoubles];
-    const int J = blockIdx.x, I = blockIdx.y;
-    if (I < J || I == k || J == k) return;
-    double acc[4][4];
-    tile_product(cbuf + static_cast<long>(I) * kSweepB * kSweepB, kSweepB, rbuf + static_cast<long>(J) * kSweepB, N,
-                 acc, buf);
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        double* row = m + (static_cast<long>(I) * kSweepB + ty * 4 + a) * N + static_cast<long>(J) * kSweepB + tx * 4;
-        double2 v0 = *reinterpret_cast<double2*>(row), v1 = *reinterpret_cast<double2*>(row + 2);
-        v0.x -= acc[a][0];
-        v0.y -= acc[a][1];
-        v1.x -= acc[a][2];
-        v1.y -= acc[a][3];
-        *reinterpret_cast<double2*>(row) = v0;
-        *reinterpret_cast<double2*>(row + 2) = v1;
+        for (int b = 0; b < 4; ++b) as[(ty * 4 + a) * LD + tx * 4 + b] = acc[a][b];  // C_I^T
+    __syncthreads();
+    for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x) {
+        const int r = q / kSweepB, c = q % kSweepB;
+        cbuf[static_cast<long>(r) * N + static_cast<long>(I) * kSweepB + c] = as[r * LD + c];
+        if (I < k) m[at_kI + static_cast<long>(r) * N + c] = as[r * LD + c];
+        else m[at_Ik + static_cast<long>(r) * N + c] = as[c * LD + r];
     }
 }
 
-// The swept pivot row and column: A_Ik = C_I (stored as A_kI = C_I^T above the diagonal), A_kk = -P.
-__global__ void __launch_bounds__(256) sweep_finish_kernel(double* __restrict__ m, int N, int k,
-                                                           const double* __restrict__ pinv,
-                                                           const double* __restrict__ cbuf) {
-    const int I = blockIdx.x;
-    for (int q = threadIdx.x; q < kSweepB * kSweepB; q += blockDim.x) {
-        const int r = q / kSweepB, c = q % kSweepB;
-        if (I == k) {
-            m[(static_cast<long>(k) * kSweepB + r) * N + static_cast<long>(k) * kSweepB + c] = -pinv[q];
-        } else if (I > k) {
-            m[(static_cast<long>(I) * kSweepB + r) * N + static_cast<long>(k) * kSweepB + c] =
-                cbuf[(static_cast<long>(I) * kSweepB + r) * kSweepB + c];
-        } else {
-            m[(static_cast<long>(k) * kSweepB + c) * N + static_cast<long>(I) * kSweepB + r] =
-                cbuf[(static_cast<long>(I) * kSweepB + r) * kSweepB + c];
+__device__ __forceinline__ void sweep_copy16(double* smem, const double* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(smem))),
+                 "l"(gmem)
+                 : "memory");
+}
+
+// A_IJ -= C_I A_kJ for the tiles (128 rows x 64 columns, row block I of two blocks) that meet the lower block
+// triangle, blocks k left alone. Bound by the FP64 pipe (n^2 kSweepB / 2 multiply-adds a step) with the tile's
+// read and write beside it: both operands sit k-major in shared memory (96 KB, two blocks an SM, so one
+// block's copies run under the other's arithmetic), and a thread's 8 x 4 patch takes 6 16-byte
+// shared-memory loads per 32 multiply-adds. Tile t of the list: I(I + 1) <= t, J = t - I(I + 1).
+constexpr std::size_t kUpdateSmem = sizeof(double) * kSweepB * (kSweepRows + kSweepB);
+
+__global__ void __launch_bounds__(256, 2) sweep_update_kernel(double* __restrict__ m, int N, int k,
+                                                             const double* __restrict__ cbuf,
+                                                             const double* __restrict__ rbuf,
+                                                             double* __restrict__ pinv_next, int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    double* xs = reinterpret_cast<double*>(sweep_smem);  // C_I^T, 64 x 128
+    double* ys = xs + kSweepB * kSweepRows;              // A_kJ, 64 x 64
+    const int T = N / kSweepB;
+    // The tile that holds the next pivot block goes first.
+    const int next = k + 1;
+    const int first = next < T ? (next / 2) * (next / 2 + 1) + next : 0;
+    const int t = static_cast<int>(blockIdx.x) == 0 ? first : (static_cast<int>(blockIdx.x) == first ? 0 : blockIdx.x);
+    int I = static_cast<int>((sqrt(4.0 * t + 1.0) - 1.0) * 0.5);
+    while (I * (I + 1) > t) --I;
+    while ((I + 1) * (I + 2) <= t) ++I;
+    const int J = t - I * (I + 1);
+    const bool pivot = next < T && t == first;
+    if (J >= T || J == k) return;  // (never the pivot's tile: its J is k + 1 < T)
+    const bool half1 = 2 * I + 1 < T;
+    for (int q = threadIdx.x; q < kSweepB * (kSweepRows / 2); q += blockDim.x) {
+        const int r = q / (kSweepRows / 2), c = q % (kSweepRows / 2) * 2;
+        if (c < kSweepB || half1)
+            sweep_copy16(xs + r * kSweepRows + c, cbuf + static_cast<long>(r) * N + static_cast<long>(I) * kSweepRows + c);
+    }
+    for (int q = threadIdx.x; q < kSweepB * (kSweepB / 2); q += blockDim.x) {
+        const int r = q / (kSweepB / 2), c = q % (kSweepB / 2) * 2;
+        sweep_copy16(ys + r * kSweepB + c, rbuf + static_cast<long>(r) * N + static_cast<long>(J) * kSweepB + c);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // A thread's rows: 4 ty .. 4 ty + 3 of both 64-row halves.
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+    double acc[2][4][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) acc[h][a][b] = 0.0;
+#pragma unroll 4
+    for (int kk = 0; kk < kSweepB; ++kk) {
+        const double2 y0 = *reinterpret_cast<const double2*>(ys + kk * kSweepB + tx * 4);
+        const double2 y1 = *reinterpret_cast<const double2*>(ys + kk * kSweepB + tx * 4 + 2);
+        const double yb[4] = {y0.x, y0.y, y1.x, y1.y};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const double* x = xs + kk * kSweepRows + h * kSweepB + ty * 4;
+            const double2 x0 = *reinterpret_cast<const double2*>(x), x1 = *reinterpret_cast<const double2*>(x + 2);
+            const double xa[4] = {x0.x, x0.y, x1.x, x1.y};
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[h][a][b] = fma(xa[a], yb[b], acc[h][a][b]);
         }
+    }
+    if (pivot) __syncthreads();  // xs is about to hold the pivot block
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int bi = 2 * I + h;
+        if (bi >= T || bi == k || bi < J) continue;  // bi < J: above the block diagonal
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            double* row = m + (static_cast<long>(bi) * kSweepB + ty * 4 + a) * N + static_cast<long>(J) * kSweepB + tx * 4;
+            double2 v0 = *reinterpret_cast<double2*>(row), v1 = *reinterpret_cast<double2*>(row + 2);
+            v0.x -= acc[h][a][0];
+            v0.y -= acc[h][a][1];
+            v1.x -= acc[h][a][2];
+            v1.y -= acc[h][a][3];
+            *reinterpret_cast<double2*>(row) = v0;
+            *reinterpret_cast<double2*>(row + 2) = v1;
+            if (pivot && bi == next) {
+                double* p = xs + (ty * 4 + a) * (kSweepB + 1) + tx * 4;
+                p[0] = v0.x;
+                p[1] = v0.y;
+                p[2] = v1.x;
+                p[3] = v1.y;
+            }
+        }
+    }
+    if (pivot) {
+        __syncthreads();
+        invert_block(xs, reinterpret_cast<double (*)[kSweepB]>(ys), pinv_next, status);
     }
 }
 
@@ -941,19 +1012,28 @@ static void dense_inverse(const DevCsr<double>& a, DevArray<double>& inv, DevArr
     const int n = a.n;
     const int T = (n + kSweepB - 1) / kSweepB;
     const int N = T * kSweepB;
-    DevArray<double> m(static_cast<std::size_t>(N) * N), pinv(kSweepB * kSweepB),
+    DevArray<double> m(static_cast<std::size_t>(N) * N), pinv(2 * kSweepB * kSweepB),
         cbuf(static_cast<std::size_t>(N) * kSweepB), rbuf(static_cast<std::size_t>(N) * kSweepB);
     m.zero(s);
     densify_lower_kernel<<<grid_for(N), kBlock, 0, s>>>(a.ptr.get(), a.col.get(), a.val.get(), n, N, m.get());
     count_launch();
     DevArray<int> status(1);
     status.zero(s);
+    constexpr std::size_t panel_smem = sizeof(double) * kSweepB * (2 * kSweepB + 2);
+    CUNIBS_CHECK(cudaFuncSetAttribute(sweep_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(panel_smem)));
+    CUNIBS_CHECK(cudaFuncSetAttribute(sweep_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(kUpdateSmem)));
+    sweep_pivot_kernel<<<1, 256, 0, s>>>(m.get(), N, pinv.get(), status.get());
+    count_launch();
+    const int TI = (T + 1) / 2;
     for (int k = 0; k < T; ++k) {
-        sweep_pivot_kernel<<<1, 256, 0, s>>>(m.get(), N, k, pinv.get(), status.get());
-        sweep_panel_kernel<<<T, 256, 0, s>>>(m.get(), N, k, pinv.get(), cbuf.get(), rbuf.get());
-        sweep_update_kernel<<<dim3(T, T), 256, 0, s>>>(m.get(), N, k, cbuf.get(), rbuf.get());
-        sweep_finish_kernel<<<T, 256, 0, s>>>(m.get(), N, k, pinv.get(), cbuf.get());
-        count_launch(4);
+        double* p = pinv.get() + (k & 1) * kSweepB * kSweepB;
+        double* p_next = pinv.get() + ((k + 1) & 1) * kSweepB * kSweepB;
+        sweep_panel_kernel<<<T, 256, panel_smem, s>>>(m.get(), N, k, p, cbuf.get(), rbuf.get());
+        sweep_update_kernel<<<TI * (TI + 1), 256, kUpdateSmem, s>>>(m.get(), N, k, cbuf.get(), rbuf.get(), p_next,
+                                                                    status.get());
+        count_launch(2);
     }
     CUNIBS_LAUNCH_CHECK("dense inverse");
     if (read_scalar(status.get(), s)) fail(kEInternal, std::string(what) + " is not positive definite");
