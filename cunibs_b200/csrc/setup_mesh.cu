@@ -266,10 +266,10 @@ __global__ void segment_starts_kernel(const int* __restrict__ sorted_keys, std::
     ptr[i] = static_cast<int>(lo);
 }
 
-// Element-pair keys for the stiffness pattern: (row node << 32) | col node, with the value
-// e*16 + i*4 + j naming the element entry. A stable sort by key groups each CSR entry's
+// Element-pair keys for the stiffness pattern: (row node << node_bits) | col node (only the bits that nodes
+// take: the sort makes a pass for every eight of them), with the value e*16 + i*4 + j naming the element entry. A stable sort by key groups each CSR entry's
 // contributions in ascending element order.
-__global__ void pair_keys_kernel(const int* __restrict__ tets, int m, std::uint64_t* __restrict__ keys,
+__global__ void pair_keys_kernel(const int* __restrict__ tets, int m, int node_bits, std::uint64_t* __restrict__ keys,
                                  int* __restrict__ vals) {
     const std::int64_t q = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= 16 * static_cast<std::int64_t>(m)) return;
@@ -278,7 +278,7 @@ __global__ void pair_keys_kernel(const int* __restrict__ tets, int m, std::uint6
     const int j = static_cast<int>(q & 3);
     const std::uint64_t r = static_cast<std::uint32_t>(tets[4 * static_cast<std::int64_t>(e) + i]);
     const std::uint64_t c = static_cast<std::uint32_t>(tets[4 * static_cast<std::int64_t>(e) + j]);
-    keys[q] = (r << 32) | c;
+    keys[q] = (r << node_bits) | c;
     vals[q] = static_cast<int>(q);
 }
 
@@ -289,13 +289,13 @@ __global__ void head_flags_kernel(const std::uint64_t* __restrict__ keys, std::i
 
 // For every run head: its entry index, column, and where its contributions start.
 __global__ void pattern_fill_kernel(const std::uint64_t* __restrict__ keys, const int* __restrict__ flags,
-                                    const int* __restrict__ pos, std::int64_t len, int* __restrict__ col,
+                                    const int* __restrict__ pos, std::int64_t len, int node_bits, int* __restrict__ col,
                                     int* __restrict__ row_of, int* __restrict__ contrib_ptr) {
     const std::int64_t q = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= len || !flags[q]) return;
     const int p = pos[q];
-    col[p] = static_cast<int>(keys[q] & 0xffffffffu);
-    row_of[p] = static_cast<int>(keys[q] >> 32);
+    col[p] = static_cast<int>(keys[q] & ((std::uint64_t{1} << node_bits) - 1));
+    row_of[p] = static_cast<int>(keys[q] >> node_bits);
     contrib_ptr[p] = static_cast<int>(q);
 }
 
@@ -566,9 +566,10 @@ void build_mesh(Mesh& m, const double* nodes_mm, int n_nodes, const int* tets, c
         const std::int64_t Q = 16 * M;
         DevArray<std::uint64_t> pk(Q), pk_sorted(Q);
         DevArray<int> pv(Q);
-        pair_keys_kernel<<<grid_for(Q), kBlock, 0, s>>>(m.tets.get(), n_tets, pk.get(), pv.get()); count_launch();
+        const int node_bits = bits_for(n_nodes);
+        pair_keys_kernel<<<grid_for(Q), kBlock, 0, s>>>(m.tets.get(), n_tets, node_bits, pk.get(), pv.get()); count_launch();
         m.contrib_idx.resize(Q);
-        sort_pairs(pk.get(), pk_sorted.get(), pv.get(), m.contrib_idx.get(), Q, 32 + bits_for(n_nodes), s);
+        sort_pairs(pk.get(), pk_sorted.get(), pv.get(), m.contrib_idx.get(), Q, 2 * node_bits, s);
         DevArray<int> flags(Q + 1), pos(Q + 1);
         head_flags_kernel<<<grid_for(Q), kBlock, 0, s>>>(pk_sorted.get(), Q, flags.get()); count_launch();
         CUNIBS_CHECK(cudaMemsetAsync(flags.get() + Q, 0, sizeof(int), s));
@@ -578,7 +579,7 @@ void build_mesh(Mesh& m, const double* nodes_mm, int n_nodes, const int* tets, c
         m.k_col.resize(nnz);
         m.contrib_ptr.resize(nnz + 1);
         DevArray<int> row_of(nnz);
-        pattern_fill_kernel<<<grid_for(Q), kBlock, 0, s>>>(pk_sorted.get(), flags.get(), pos.get(), Q, m.k_col.get(),
+        pattern_fill_kernel<<<grid_for(Q), kBlock, 0, s>>>(pk_sorted.get(), flags.get(), pos.get(), Q, node_bits, m.k_col.get(),
                                                            row_of.get(), m.contrib_ptr.get()); count_launch();
         const int q_end = static_cast<int>(Q);
         CUNIBS_CHECK(cudaMemcpyAsync(m.contrib_ptr.get() + nnz, &q_end, sizeof(int), cudaMemcpyHostToDevice, s));
