@@ -540,68 +540,69 @@ __global__ void __launch_bounds__(32 * kFitWarps) harmonic_weights_kernel(const 
     if (lane == 0) status[s] = rung;
 }
 
+// The harmonic apply's entries in flight: eight where the GPU holds every thread (148 SMs of 2048), so that
+// registers cost nothing (one placement on 121k nodes: the apply 53 us at one entry); two where they queue.
+constexpr std::int64_t kFewThreads = 148 * 2048;
+constexpr int kEntriesFew = 8;
+constexpr int kEntriesMany = 2;
+
 // --- apply ------------------------------------------------------------------------------------
 
-// Harmonic: E_s = -sum_p w_p v_m - dA/dt(node), FP64 accumulation in patch order; one thread per
-// (slot, column), K column threads of a slot adjacent so the operator entry is one broadcast load.
-__global__ void harmonic_apply_kernel(const float4* __restrict__ wq, const int* __restrict__ pptr,
-                                      const int* __restrict__ slot_node, int n_slots, const double* __restrict__ x,
-                                      int K, int ground, const float* __restrict__ dadt_nodes, int n_nodes, int k,
-                                      float* __restrict__ e_slots) {
+// Harmonic: E_s = -sum_p w_p v_m - dA/dt(node), FP64 accumulation in patch order; one thread per slot and
+// C adjacent columns (C = 2 where K is even: one operator load serves both and the potential pair is one
+// 16-byte gather), a slot's threads adjacent so that the operator entry is one broadcast load. The walk of a
+// patch is a chain of loads (entry, then potential), bound by its latency: U entries' loads are issued before
+// their multiply-adds, which stay in patch order, so the result depends on neither C nor U.
+template <int C, int U>
+__global__ void __launch_bounds__(kBlock) harmonic_apply_kernel(const float4* __restrict__ wq,
+                                                                const int* __restrict__ pptr,
+                                                                const int* __restrict__ slot_node, int n_slots,
+                                                                const double* __restrict__ x, int K, int ground,
+                                                                const float* __restrict__ dadt_nodes, int n_nodes,
+                                                                int k, float* __restrict__ e_slots) {
     const std::int64_t q = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int s = static_cast<int>(q / K), c = static_cast<int>(q % K);
-    if (s >= n_slots || c >= k) return;
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    for (int p = pptr[s], end = pptr[s + 1]; p < end; ++p) {
-        const float4 e = wq[p];
-        const int m = __float_as_int(e.w);
-        const double vm = (m == ground) ? 0.0 : x[static_cast<std::int64_t>(m - (m > ground ? 1 : 0)) * K + c];
-        ax = fma(static_cast<double>(e.x), vm, ax);
-        ay = fma(static_cast<double>(e.y), vm, ay);
-        az = fma(static_cast<double>(e.z), vm, az);
-    }
-    const int node = slot_node[s];
-    const float* da = dadt_nodes + (static_cast<std::int64_t>(c) * n_nodes + node) * 3;
-    float* o = e_slots + (static_cast<std::int64_t>(c) * n_slots + s) * 3;
-    o[0] = static_cast<float>(-ax - static_cast<double>(da[0]));
-    o[1] = static_cast<float>(-ay - static_cast<double>(da[1]));
-    o[2] = static_cast<float>(-az - static_cast<double>(da[2]));
-}
-
-// The same with one thread per (slot, column pair): one operator load serves both columns and the
-// potential pair is one 16-byte gather; each column's sums are bitwise the one-column kernel's.
-__global__ void harmonic_apply_pair_kernel(const float4* __restrict__ wq, const int* __restrict__ pptr,
-                                           const int* __restrict__ slot_node, int n_slots,
-                                           const double* __restrict__ x, int K, int ground,
-                                           const float* __restrict__ dadt_nodes, int n_nodes, int k,
-                                           float* __restrict__ e_slots) {
-    const std::int64_t q = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int L = K / 2;
-    const int s = static_cast<int>(q / L), c0 = 2 * static_cast<int>(q % L);
+    const int L = K / C;
+    const int s = static_cast<int>(q / L), c0 = C * static_cast<int>(q % L);
     if (s >= n_slots || c0 >= k) return;
-    const double2* xv = reinterpret_cast<const double2*>(x);
-    double ax0 = 0.0, ay0 = 0.0, az0 = 0.0, ax1 = 0.0, ay1 = 0.0, az1 = 0.0;
-    for (int p = pptr[s], end = pptr[s + 1]; p < end; ++p) {
-        const float4 e = wq[p];
-        const int m = __float_as_int(e.w);
-        const double2 vm = (m == ground) ? make_double2(0.0, 0.0)
-                                         : xv[static_cast<std::int64_t>(m - (m > ground ? 1 : 0)) * L + c0 / 2];
-        ax0 = fma(static_cast<double>(e.x), vm.x, ax0);
-        ay0 = fma(static_cast<double>(e.y), vm.x, ay0);
-        az0 = fma(static_cast<double>(e.z), vm.x, az0);
-        ax1 = fma(static_cast<double>(e.x), vm.y, ax1);
-        ay1 = fma(static_cast<double>(e.y), vm.y, ay1);
-        az1 = fma(static_cast<double>(e.z), vm.y, az1);
+    double acc[C][3] = {};
+    const int end = pptr[s + 1];
+    for (int p = pptr[s]; p < end; p += U) {
+        float4 e[U];
+        double v[U][C];
+#pragma unroll
+        for (int u = 0; u < U; ++u) e[u] = wq[p + u < end ? p + u : end - 1];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int m = __float_as_int(e[u].w);
+            const std::int64_t at = static_cast<std::int64_t>(m - (m > ground ? 1 : 0)) * L + c0 / C;
+            if constexpr (C == 2) {
+                const double2 d = m == ground ? make_double2(0.0, 0.0) : reinterpret_cast<const double2*>(x)[at];
+                v[u][0] = d.x;
+                v[u][1] = d.y;
+            } else {
+                v[u][0] = m == ground ? 0.0 : x[at];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (p + u < end) {
+#pragma unroll
+                for (int h = 0; h < C; ++h) {
+                    acc[h][0] = fma(static_cast<double>(e[u].x), v[u][h], acc[h][0]);
+                    acc[h][1] = fma(static_cast<double>(e[u].y), v[u][h], acc[h][1]);
+                    acc[h][2] = fma(static_cast<double>(e[u].z), v[u][h], acc[h][2]);
+                }
+            }
     }
     const int node = slot_node[s];
-    const double a[2][3] = {{ax0, ay0, az0}, {ax1, ay1, az1}};
-    for (int h = 0; h < 2 && c0 + h < k; ++h) {
+#pragma unroll
+    for (int h = 0; h < C; ++h) {
         const int c = c0 + h;
+        if (c >= k) break;
         const float* da = dadt_nodes + (static_cast<std::int64_t>(c) * n_nodes + node) * 3;
         float* o = e_slots + (static_cast<std::int64_t>(c) * n_slots + s) * 3;
-        o[0] = static_cast<float>(-a[h][0] - static_cast<double>(da[0]));
-        o[1] = static_cast<float>(-a[h][1] - static_cast<double>(da[1]));
-        o[2] = static_cast<float>(-a[h][2] - static_cast<double>(da[2]));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) o[a] = static_cast<float>(-acc[h][a] - static_cast<double>(da[a]));
     }
 }
 
@@ -826,17 +827,19 @@ void apply_recovery(const Mesh& m, const RecoveryOp& op, const double* x_red, in
                     const float* e_elem, int k, float* e_slots, float* E, float* magn, cudaStream_t s) {
     if (op.mode == kRecHarmonic) {
         const char* lanes = std::getenv("CUNIBS_LANE_COLUMNS");
-        if (K % 2 == 0 && !(lanes != nullptr && lanes[0] == '1')) {
-            const std::int64_t n = static_cast<std::int64_t>(op.n_slots) * (K / 2);
-            harmonic_apply_pair_kernel<<<grid_for(n), kBlock, 0, s>>>(op.wq.get(), op.ptr.get(), op.slot_node.get(),
-                                                                      op.n_slots, x_red, K, m.ground, dadt_nodes,
-                                                                      m.n_nodes, k, e_slots);
-        } else {
-            const std::int64_t n = static_cast<std::int64_t>(op.n_slots) * K;
-            harmonic_apply_kernel<<<grid_for(n), kBlock, 0, s>>>(op.wq.get(), op.ptr.get(), op.slot_node.get(),
-                                                                 op.n_slots, x_red, K, m.ground, dadt_nodes, m.n_nodes,
-                                                                 k, e_slots);
-        }
+        const int C = K % 2 == 0 && !(lanes != nullptr && lanes[0] == '1') ? 2 : 1;
+        const std::int64_t n = static_cast<std::int64_t>(op.n_slots) * (K / C);
+        auto go = [&](auto cc, auto uc) {
+            harmonic_apply_kernel<decltype(cc)::value, decltype(uc)::value><<<grid_for(n), kBlock, 0, s>>>(
+                op.wq.get(), op.ptr.get(), op.slot_node.get(), op.n_slots, x_red, K, m.ground, dadt_nodes, m.n_nodes,
+                k, e_slots);
+        };
+        auto pick = [&](auto cc) {
+            if (n < kFewThreads) go(cc, std::integral_constant<int, kEntriesFew>{});
+            else go(cc, std::integral_constant<int, kEntriesMany>{});
+        };
+        if (C == 2) pick(std::integral_constant<int, 2>{});
+        else pick(std::integral_constant<int, 1>{});
     } else {
         const bool nodes = op.mode == kRecSprGlobal;
         const std::int64_t n = static_cast<std::int64_t>(op.n_slots) * k;

@@ -1101,13 +1101,6 @@ __global__ void __launch_bounds__(tile_threads<K>()) cheby_dot_kernel(
     if (last_block(counter)) finish_beta<K>(partials, rz, frozen, beta);
 }
 
-// r_lo = r rounded to the V-cycle's type (the first V-cycle input of FP64 PCG over an FP32 V-cycle).
-template <typename T, typename TZ>
-__global__ void narrow_kernel(std::int64_t count, const T* __restrict__ r, TZ* __restrict__ r_lo) {
-    const std::int64_t q = static_cast<std::int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (q < count) r_lo[q] = static_cast<TZ>(r[q]);
-}
-
 // Mixed refinement outer step: R = B - A X in FP64; r32 = (float)R; per column the true relative
 // residual, the outer freeze, the inner solve's reference norm, its starting freeze, and the
 // inner target: reduce the residual by eta = max(eta_min, 0.3 * tol / rel), just enough (with a
@@ -1418,22 +1411,23 @@ class Solver {
         while_unsupported = true;
         return false;
     }
+    // b: the right-hand sides (n, K); a warm start's guess is in X.
     template <int K, typename TZ>
-    void solve_plain(int k, const Params& prm, SolveStats& st, bool warm);
+    void solve_plain(const double* b, int k, const Params& prm, SolveStats& st, bool warm);
     template <int K>
     void solve_mixed(int k, const Params& prm, SolveStats& st, bool warm);
     // R = B - A X in FP64 for a warm start, then the per-column zero-guess fallback.
     template <int K>
-    void warm_residual(const DevCsr<double>& A) {
+    void warm_residual(const DevCsr<double>& A, const double* b) {
         constexpr int TT = tile_threads<K>();
         dispatch_tpr<K>(tpr0(), [&](auto tc) {
             constexpr int TPR = decltype(tc)::value;
             residual64_kernel<K, TPR><<<(n + ReduceTile<TPR>::kRows - 1) / ReduceTile<TPR>::kRows, TT, 0, stream>>>(
-                n, A.ptr.get(), A.col.get(), A.val.get(), B.get(), X.get(), R.get());
+                n, A.ptr.get(), A.col.get(), A.val.get(), b, X.get(), R.get());
         });
         norm2_kernel<double, K><<<reduce_grid(n), TT, 0, stream>>>(n, R.get(), partials.get(), counter.get(),
                                                                   r0sq.get());
-        guess_fallback_kernel<K><<<n_tiles(n), TT, 0, stream>>>(n, X.get(), R.get(), B.get(), ref_sq.get(),
+        guess_fallback_kernel<K><<<n_tiles(n), TT, 0, stream>>>(n, X.get(), R.get(), b, ref_sq.get(),
                                                                 r0sq.get(), init_rel.get());
         count_launch(3);
     }
@@ -1715,23 +1709,67 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
     return fuse_dot && deg >= 2;
 }
 
-// Before a first tail: p = 0 and rz = 1, so beta is finite and p becomes z.
-// Per-column start of a PCG solve: a zero right-hand side column starts (and stays) frozen at
-// iteration 0, so the loop never waits on it; the host reports it after the solve.
-__global__ void start_columns_kernel(const double* __restrict__ ref_sq, int K, int max_iters, int* __restrict__ frozen,
-                                     int* __restrict__ conv_iter, double* __restrict__ rel) {
-    const int c = threadIdx.x;
-    if (c < K) {
-        const bool live = ref_sq[c] > 0.0;
-        frozen[c] = live ? 0 : 1;
-        conv_iter[c] = live ? max_iters : 0;
-        rel[c] = 0.0;
-    }
-}
-
 __global__ void fill_kernel(double* v, int n, double x) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) v[i] = x;
+}
+
+// Everything a PCG solve starts from, in one pass: p = 0 and Ap = 0 (with rz = 1, so that the first beta is finite
+// and p becomes z), the residual rounded to the V-cycle's type (r_lo, when it is narrower), the V-cycle's
+// first smoothing step z0 = alpha0 dinv r, and per column the state of the loop. From a zero guess also
+// x = 0, r = b and ref_sq = ||b||^2 (the last block finishes); a warm start has formed x, r and ref_sq. A
+// zero right-hand side column starts (and stays) frozen at iteration 0, so the loop never waits on it; the
+// host reports it after the solve.
+template <typename TZ, int K, bool WARM>
+__global__ void __launch_bounds__(tile_threads<K>()) start_kernel(
+    int n, const double* __restrict__ b, double* __restrict__ x, double* __restrict__ r, double* __restrict__ p,
+    double* __restrict__ ap, TZ* __restrict__ r_lo, const TZ* __restrict__ dinv, TZ alpha0, TZ* __restrict__ z0,
+    double* partials, unsigned* counter, double* __restrict__ ref_sq, int max_iters, double tol,
+    int* __restrict__ frozen, int* __restrict__ conv_iter, double* __restrict__ rel, double* __restrict__ rz,
+    double* __restrict__ tol_vec, int* __restrict__ iter_counter, int* __restrict__ cap) {
+    const int slot = threadIdx.x / K;
+    const int c = threadIdx.x % K;
+    const int tiles = n_tiles_dev(n);
+    double v = 0.0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int row = t * kTileRows + slot;
+        if (row < n) {
+            const long q = static_cast<long>(row) * K + c;
+            double rq;
+            if constexpr (WARM) {
+                rq = r[q];
+            } else {
+                rq = b[q];
+                x[q] = 0.0;
+                r[q] = rq;
+                v += rq * rq;
+            }
+            p[q] = 0.0;
+            ap[q] = 0.0;
+            const TZ rl = static_cast<TZ>(rq);
+            if (r_lo != nullptr) r_lo[q] = rl;
+            if (z0 != nullptr) z0[q] = alpha0 * dinv[row] * rl;
+        }
+    }
+    if constexpr (!WARM) block_partial<K>(v, partials);
+    if (last_block(counter)) {
+        __shared__ double tot[K];
+        if constexpr (!WARM) final_reduce<K>(partials, gridDim.x, tot);
+        if (threadIdx.x < K) {
+            const int cc = threadIdx.x;
+            if constexpr (!WARM) ref_sq[cc] = tot[cc];
+            const bool live = ref_sq[cc] > 0.0;
+            frozen[cc] = live ? 0 : 1;
+            conv_iter[cc] = live ? max_iters : 0;
+            rel[cc] = 0.0;
+            rz[cc] = 1.0;
+            tol_vec[cc] = tol;
+        }
+        if (threadIdx.x == 0) {
+            *iter_counter = 0;
+            *cap = max_iters;
+        }
+    }
 }
 
 template <typename TZ, int K>
@@ -1768,7 +1806,7 @@ void Solver::pcg_iteration(const int* ptr, const int* col, const T* val, T* x, T
 }
 
 template <int K, typename TZ>
-void Solver::solve_plain(int k, const Params& prm, SolveStats& st, bool warm) {
+void Solver::solve_plain(const double* b, int k, const Params& prm, SolveStats& st, bool warm) {
     constexpr bool narrow = !std::is_same<TZ, double>::value;
     TZ* rv = nullptr;
     TZ* zv = nullptr;
@@ -1781,33 +1819,30 @@ void Solver::solve_plain(int k, const Params& prm, SolveStats& st, bool warm) {
     }
     const int key = narrow ? 4 : 2;
     constexpr int TT = tile_threads<K>();
-    const unsigned g = n_tiles(n);
     cudaStream_t s = stream;
     const DevCsr<double>& A = h->levels.empty() ? h->coarse : h->levels[0].a;
-    const std::size_t nk = static_cast<std::size_t>(n) * K;
-    norm2_kernel<double, K><<<reduce_grid(n), TT, 0, s>>>(n, B.get(), partials.get(), counter.get(), ref_sq.get()); count_launch();
-    if (warm) {
-        warm_residual<K>(A);
-    } else {
-        X.zero(s);
-        CUNIBS_CHECK(cudaMemcpyAsync(R.get(), B.get(), nk * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    }
-    iter_counter.zero(s);
-    P.zero(s);
-    AP.zero(s);  // the first iteration's Ap = A z + beta Ap reads it
-    start_columns_kernel<<<1, 32, 0, s>>>(ref_sq.get(), K, prm.max_iters, frozen.get(), conv_iter.get(), rel.get());
-    count_launch();
-    fill_kernel<<<1, 32, 0, s>>>(rz.get(), K, 1.0);
-    fill_kernel<<<1, 32, 0, s>>>(tolv.get(), K, prm.tolerance);
-    count_launch(2);
-    if constexpr (narrow) {
-        const std::int64_t count = static_cast<std::int64_t>(n) * K;
-        narrow_kernel<double, TZ><<<grid_for(count), kBlock, 0, s>>>(count, R.get(), rv);
+    // The V-cycle's first smoothing step is its finest level's; without levels it is the dense solve alone.
+    const bool has_levels = !h->levels.empty();
+    TZ* z0 = has_levels && h->vcycle_levels > 0 ? first0<TZ>() : nullptr;
+    const TZ* dinv0 = has_levels ? ldinv<TZ>(0) : nullptr;
+    auto start = [&](auto warm_c) {
+        start_kernel<TZ, K, decltype(warm_c)::value><<<reduce_grid(n), TT, 0, s>>>(
+            n, b, X.get(), R.get(), P.get(), AP.get(), narrow ? rv : nullptr, dinv0,
+            static_cast<TZ>(h->cheby.alpha0), z0, partials.get(), counter.get(), ref_sq.get(), prm.max_iters,
+            prm.tolerance, frozen.get(), conv_iter.get(), rel.get(), rz.get(), tolv.get(), iter_counter.get(),
+            cap.get());
         count_launch();
+    };
+    if (warm) {
+        norm2_kernel<double, K><<<reduce_grid(n), TT, 0, s>>>(n, b, partials.get(), counter.get(), ref_sq.get());
+        count_launch();
+        warm_residual<K>(A, b);
+        start(std::true_type{});
+    } else {
+        start(std::false_type{});
     }
-    pcg_tail<TZ, K>(rv, zv, false);
+    pcg_tail<TZ, K>(rv, zv, z0 != nullptr);
     int it = 0;
-    set_cap(prm.max_iters);
     long long nodes = 0;
     const bool device_loop = run_while({key, K, 0}, [&](cudaGraphConditionalHandle hnd) {
         pcg_iteration<double, TZ, K>(A.ptr.get(), A.col.get(), A.val.get(), X.get(), R.get(), P.get(), AP.get(), rv,
@@ -1853,7 +1888,7 @@ void Solver::solve_mixed(int k, const Params& prm, SolveStats& st, bool warm) {
     DevArray<float> coarse32;
     if (A32 == nullptr) fail(kEInval, "mixed precision needs at least one AMG level");
     norm2_kernel<double, K><<<reduce_grid(n), TT, 0, s>>>(n, B.get(), partials.get(), counter.get(), ref_sq.get()); count_launch();
-    if (warm) warm_residual<K>(A);
+    if (warm) warm_residual<K>(A, B.get());
     outer_conv.zero(s);
     iter_counter.zero(s);
     CUNIBS_CHECK(cudaMemcpyAsync(h_dbl, ref_sq.get(), sizeof(double) * K, cudaMemcpyDeviceToHost, s));
@@ -1975,12 +2010,16 @@ void solver_solve(Solver& sv, const double* Bin, double* Xout, int k, int K, con
         CUNIBS_CHECK(cudaEventRecord(ev, s));
         CUNIBS_CHECK(cudaStreamWaitEvent(sv.stream, ev, 0));
         const std::size_t nk = static_cast<std::size_t>(sv.n) * KK;
-        CUNIBS_CHECK(cudaMemcpyAsync(sv.B.get(), Bin, nk * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream));
         if (X0) CUNIBS_CHECK(cudaMemcpyAsync(sv.X.get(), X0, nk * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream));
-        else sv.X.zero(sv.stream);
-        if (prm.precision == kMixed) sv.solve_mixed<KK>(k, prm, st, X0 != nullptr);
-        else if (prm.precision == kFp64CgFp32Mg) sv.solve_plain<KK, float>(k, prm, st, X0 != nullptr);
-        else sv.solve_plain<KK, double>(k, prm, st, X0 != nullptr);
+        if (prm.precision == kMixed) {
+            CUNIBS_CHECK(cudaMemcpyAsync(sv.B.get(), Bin, nk * sizeof(double), cudaMemcpyDeviceToDevice, sv.stream));
+            if (!X0) sv.X.zero(sv.stream);
+            sv.solve_mixed<KK>(k, prm, st, X0 != nullptr);
+        } else if (prm.precision == kFp64CgFp32Mg) {
+            sv.solve_plain<KK, float>(Bin, k, prm, st, X0 != nullptr);
+        } else {
+            sv.solve_plain<KK, double>(Bin, k, prm, st, X0 != nullptr);
+        }
         if (X0)
             CUNIBS_CHECK(cudaMemcpyAsync(sv.h_dbl + 3 * KK, sv.init_rel.get(), sizeof(double) * KK,
                                          cudaMemcpyDeviceToHost, sv.stream));

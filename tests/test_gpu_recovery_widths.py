@@ -1,0 +1,32 @@
+"""The harmonic recovery at every block width against the oracle's mirror of its arithmetic, bit for bit: one
+column or pairs a thread, few threads (eight patch entries in flight) or many. Needs a B200."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from cunibs_b200 import _native
+from cunibs_b200.synthetic import sphere_head
+from oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("spacing, widths", [(12.0, (1, 2, 3, 8, 16)), (5.0, (1, 8))])
+def test_harmonic_apply_bit_exact(spacing, widths):
+    mesh = sphere_head(spacing, 90.0, jitter_mm=0.2, seed=5)
+    orc = Oracle(mesh)
+    ctx = _native.Context(mesh.nodes_mm, mesh.tet_nodes, mesh.tet_tags, mesh.skin_tris)
+    try:
+        rng = np.random.default_rng(8)
+        for k in widths:
+            v = rng.standard_normal((k, ctx.n_nodes))
+            v[:, ctx.ground_node] = 0.0
+            dadt = rng.standard_normal((k, ctx.n_nodes, 3)).astype(np.float32)
+            got = ctx.recover("harmonic", v=v, dadt_nodes=dadt)
+            want = orc.recovery_apply("harmonic", v=v, dadt_nodes=dadt)
+            for a, b, name in zip(got, want, ("E_slots", "E", "magnE")):
+                np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32), err_msg=f"{name} k={k}")
+    finally:
+        ctx.close()
