@@ -46,3 +46,21 @@ def test_solutions_and_widths(spacing, precision):
         assert (itw <= 1).all() and np.linalg.norm(xw - x16) <= 1e-8 * np.linalg.norm(x16)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("spacing", [4.2, 3.8, 3.0])
+@pytest.mark.parametrize("precision", [_native.PREC_SPLIT, _native.PREC_PLAIN_FP64])
+def test_groups_of_tiles_leave_the_sums_as_they_are(spacing, precision):
+    """More than 592 tiles of 64 rows: blocks of one, two and four columns hold several groups, 16 columns one."""
+    m = sphere_head(spacing, 90.0, jitter_mm=0.2, seed=2)
+    ctx = _native.Context(m.nodes_mm, m.tet_nodes, m.tet_tags, m.skin_tris, _native.default_params())
+    try:
+        b = np.random.default_rng(5).standard_normal((ctx.array("a_ptr", 0).shape[0] - 1, 16))
+        x16, it, rel = ctx.solve(b, 16, 16, precision=precision, tolerance=TOL)
+        assert (rel <= TOL).all()
+        for k in (1, 2, 4):
+            xk, itk, _ = ctx.solve(np.ascontiguousarray(b[:, :k]), k, k, precision=precision, tolerance=TOL)
+            np.testing.assert_array_equal(xk, x16[:, :k])
+            np.testing.assert_array_equal(itk, it[:k])
+    finally:
+        ctx.close()
