@@ -973,14 +973,9 @@ int cunibs_sigma_begin(cunibs_context* c, const double* dip_pos_m, const double*
             const BlockSlot& sl0 = c->slots[st->slot];
             DevArray<double> td;
             td.upload(tables.data(), tables.size(), s);
-            DevArray<float> wts(static_cast<std::size_t>(1 + P) * m.n_tets);
-            sigma_element_weights(m, td.get(), 1 + P, wts.get(), s);
-            const std::size_t nk = static_cast<std::size_t>(n_red) * K;
-            st->rhs.resize((1 + P) * nk);
-            for (int t = 0; t <= P; ++t)
-                rhs_block(m, sl0.dadt_elm.get(), st->k, K, st->rhs.get() + t * nk, s,
-                          wts.get() + static_cast<std::size_t>(t) * m.n_tets);
-            CUNIBS_CHECK(cudaStreamSynchronize(s));  // td and wts leave scope
+            st->rhs.resize((1 + P) * static_cast<std::size_t>(n_red) * K);
+            rhs_block_tables(m, sl0.dadt_elm.get(), st->k, K, td.get(), 1 + P, st->rhs.get(), s);
+            CUNIBS_CHECK(cudaStreamSynchronize(s));  // td leaves scope
         }
         phase(4);
         st->x_nom.resize(static_cast<std::size_t>(n_red) * K);

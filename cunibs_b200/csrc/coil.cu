@@ -301,6 +301,50 @@ __global__ void __launch_bounds__(64 * K) rhs_kernel(const float* __restrict__ e
     b_red[static_cast<long>(r) * K + c] = acc;
 }
 
+// rhs_kernel's right-hand sides for n_tables conductivity tables at once (b_red, n_tables by n_red by K), each
+// element weighed by -(vol_e table[tag_e]) in FP32: the element field and gradients are read once for all tables.
+constexpr int kMaxRhsTables = 11;
+template <int K>
+__global__ void __launch_bounds__(64 * K) rhs_tables_kernel(const float* __restrict__ elm, const float* __restrict__ g32,
+                                                            const float* __restrict__ vols32,
+                                                            const int* __restrict__ tags,
+                                                            const double* __restrict__ tables, int n_tables,
+                                                            const int* __restrict__ ptr, const int* __restrict__ idx,
+                                                            int n_nodes, int n_tets, int k, int ground,
+                                                            double* __restrict__ b_red) {
+    __shared__ float tab[kMaxRhsTables][12];
+    for (int q = threadIdx.x; q < n_tables * 11; q += blockDim.x)
+        tab[q / 11][q % 11] = static_cast<float>(tables[q]);
+    __syncthreads();
+    const int r = blockIdx.x * 64 + threadIdx.x / K;
+    const int c = threadIdx.x % K;
+    if (r >= n_nodes - 1) return;
+    const int i = r + (r >= ground ? 1 : 0);
+    const int src = c < k ? c : k - 1;
+    const float* el = elm + static_cast<long>(src) * n_tets * 3;
+    double acc[kMaxRhsTables];
+#pragma unroll
+    for (int t = 0; t < kMaxRhsTables; ++t) acc[t] = 0.0;
+    for (int q = ptr[i]; q < ptr[i + 1]; ++q) {
+        const int corner = idx[q];
+        const int e = corner >> 2;
+        const float* gc = g32 + 3 * static_cast<long>(corner);
+        const double d = static_cast<double>(el[3 * static_cast<long>(e)]) * gc[0] +
+                         static_cast<double>(el[3 * static_cast<long>(e) + 1]) * gc[1] +
+                         static_cast<double>(el[3 * static_cast<long>(e) + 2]) * gc[2];
+        const float vol = vols32[e];
+        const int tag = tags[e];
+#pragma unroll
+        for (int t = 0; t < kMaxRhsTables; ++t) {
+            if (t < n_tables) acc[t] += static_cast<double>(-(vol * tab[t][tag])) * d;
+        }
+    }
+    const long nk = static_cast<long>(n_nodes - 1) * K;
+#pragma unroll
+    for (int t = 0; t < kMaxRhsTables; ++t)
+        if (t < n_tables) b_red[t * nk + static_cast<long>(r) * K + c] = acc[t];
+}
+
 // w_ij = sum over entry (i, j)'s element contributions (ascending element) of 1/4 neg_vc[e] g[e, i]:
 // b_i = sum_{corners of i} neg_vc[e] (1/4 sum_{n in e} A_n) . g[e, i] = sum_j w_ij . A_j.
 __global__ void rhs_weights_kernel(const float* __restrict__ g32, const float* __restrict__ neg_vc,
@@ -463,14 +507,8 @@ void rhs_block_nodes(Mesh& m, const float* nodal, int k, int K, double* b_red, c
     CUNIBS_LAUNCH_CHECK("rhs from nodes");
 }
 
-void rhs_block(const Mesh& m, const float* elm, int k, int K, double* b_red, cudaStream_t s, const float* neg_vc) {
-    const unsigned g = (m.n_nodes - 1 + 63) / 64;
-    const float* w = neg_vc ? neg_vc : m.neg_vc32.get();
-    auto go = [&](auto kc) {
-        constexpr int KK = decltype(kc)::value;
-        rhs_kernel<KK><<<g, 64 * KK, 0, s>>>(elm, m.g32.get(), w, m.n2c_ptr.get(), m.n2c_idx.get(),
-                                             m.n_nodes, m.n_tets, k, m.ground, b_red); count_launch();
-    };
+template <typename F>
+static void dispatch_rhs_width(int K, F&& go) {
     switch (K) {
         case 1: go(std::integral_constant<int, 1>{}); break;
         case 2: go(std::integral_constant<int, 2>{}); break;
@@ -479,6 +517,29 @@ void rhs_block(const Mesh& m, const float* elm, int k, int K, double* b_red, cud
         case 16: go(std::integral_constant<int, 16>{}); break;
         default: fail(kEInval, "block width must be one of {1, 2, 4, 8, 16}");
     }
+}
+
+void rhs_block_tables(const Mesh& m, const float* elm, int k, int K, const double* tables_dev, int n_tables,
+                      double* b_red, cudaStream_t s) {
+    if (n_tables < 1 || n_tables > kMaxRhsTables) fail(kEInternal, "between 1 and 11 conductivity tables");
+    dispatch_rhs_width(K, [&](auto kc) {
+        constexpr int KK = decltype(kc)::value;
+        rhs_tables_kernel<KK><<<(m.n_nodes - 1 + 63) / 64, 64 * KK, 0, s>>>(
+            elm, m.g32.get(), m.vols32.get(), m.tags.get(), tables_dev, n_tables, m.n2c_ptr.get(), m.n2c_idx.get(),
+            m.n_nodes, m.n_tets, k, m.ground, b_red);
+        count_launch();
+    });
+    CUNIBS_LAUNCH_CHECK("rhs of several conductivity tables");
+}
+
+void rhs_block(const Mesh& m, const float* elm, int k, int K, double* b_red, cudaStream_t s) {
+    dispatch_rhs_width(K, [&](auto kc) {
+        constexpr int KK = decltype(kc)::value;
+        rhs_kernel<KK><<<(m.n_nodes - 1 + 63) / 64, 64 * KK, 0, s>>>(elm, m.g32.get(), m.neg_vc32.get(),
+                                                                     m.n2c_ptr.get(), m.n2c_idx.get(), m.n_nodes,
+                                                                     m.n_tets, k, m.ground, b_red);
+        count_launch();
+    });
     CUNIBS_LAUNCH_CHECK("rhs");
 }
 

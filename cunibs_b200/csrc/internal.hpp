@@ -281,7 +281,10 @@ void dadt_near_general(const Mesh& m, const float* dip_packed, int n_dip, const 
 void set_last_error(const std::string& message);
 // neg_vc: the per-element weights -(vol * sigma) in FP32 (null: the mesh's own).
 void rhs_block(const Mesh& m, const float* dadt_elm, int k, int k_pad, double* b_red /* (N-1, k_pad) */,
-               cudaStream_t s, const float* neg_vc = nullptr);
+               cudaStream_t s);
+// The right-hand sides of n_tables (1..11) conductivity tables (n_tables, 11) in one pass: b_red (n_tables, N-1, k_pad).
+void rhs_block_tables(const Mesh& m, const float* dadt_elm, int k, int k_pad, const double* tables_dev, int n_tables,
+                      double* b_red, cudaStream_t s);
 // The same right-hand side from the nodal dA/dt (k, N, 3) through the mesh's rhs_w (built here when
 // stale): equal to rhs_block of the element average up to rounding, with no element pass.
 void rhs_block_nodes(Mesh& m, const float* dadt_nodes, int k, int k_pad, double* b_red, cudaStream_t s);
@@ -419,10 +422,6 @@ struct SigmaDraw {
 };
 // Values of the finest operator for one draw: comp[0] + sum_t w_t comp[1 + t] (comp (1 + n_tags, nnz)).
 void sigma_combine(const double* comp, int n_tags, long nnz, const SigmaWeights& w, double* out, cudaStream_t s);
-// -vol of the elements of each table entry's tissue, zero elsewhere: out (n_tables, n_tets) FP32,
-// tables (n_tables, 11) of per-tag weights (the right-hand side's per-element weights of a
-// conductivity table whose entries are those weights).
-void sigma_element_weights(const Mesh& m, const double* tables_dev, int n_tables, float* out, cudaStream_t s);
 // Sensitivity right-hand sides c_t of the nominal potential x_red (n_red, K): c_out (n_red, P, K).
 void sigma_sens_rhs(const Mesh& m, const double* x_red, const float* dadt_elm, int k, int K, const SigmaSlots& slots,
                     int P, double* c_out, cudaStream_t s);
