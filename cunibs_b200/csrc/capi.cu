@@ -59,7 +59,8 @@ void cunibs::set_last_error(const std::string& message) { g_last_error = message
 // What a block's preparation (placement, dA/dt, right-hand side) leaves for its solve. Two slots
 // let the next block be prepared while the previous one is solved.
 struct BlockSlot {
-    DevArray<double> in_pos, in_mom, in_centers, in_handles, in_dists;  // host-entry inputs, uploaded
+    DevArray<double> in;          // host-entry inputs, uploaded: positions, moments, centres, handles, distances
+    double* h_in = nullptr;       // pinned (Pinned::in)
     DevArray<double> T, B, X0;  // X0: the learned initial guess
     DevArray<int> deg;
     DevArray<unsigned char> dip_packed;
@@ -67,8 +68,8 @@ struct BlockSlot {
     // Nodes the coil table does not cover, per placement (p * N + ...), and their counts.
     DevArray<int> near_list, near_cnt;
     cudaEvent_t prepared = nullptr;
-    int* h_deg = nullptr;   // pinned: the degenerate-placement flags
-    int* h_near = nullptr;  // pinned: near_cnt, copied when the block's dA/dt read the table
+    int* h_deg = nullptr;   // pinned (Pinned::deg): the degenerate-placement flags
+    int* h_near = nullptr;  // pinned (Pinned::near): near_cnt, copied when the block's dA/dt read the table
     bool near_valid = false;
 };
 
@@ -78,6 +79,19 @@ struct Staging {
     double rel[16];
     int used[16];
     double init[16];
+};
+
+constexpr int kPinnedDipoles = 4096;
+
+// A context's pinned host memory, one allocation (each cudaHostAlloc takes about 0.4 ms).
+struct Pinned {
+    Staging staging;
+    int coil_flag;
+    int deg[2][16], near[2][16];
+    double transforms[16 * 16], summary[kSummaryLen * 16];  // a finished block's small outputs
+    // Host inputs of a block on their way up, one copy instead of five from pageable memory: a coil of up to
+    // kPinnedDipoles dipoles and the placements. Larger coils are copied from where they are.
+    double in[2][6 * kPinnedDipoles + 7 * 16];
 };
 
 struct PendingBlock {
@@ -129,14 +143,17 @@ struct cunibs_context {
     std::deque<PendingBlock> pending;
     int next_slot = 0;
     long long next_ticket = 1;
-    int* h_coil_flag = nullptr;  // pinned
-    Staging* staging = nullptr;  // pinned
+    Pinned* pinned = nullptr;
+    int* h_coil_flag = nullptr;  // pinned->coil_flag
+    Staging* staging = nullptr;  // &pinned->staging
     cudaEvent_t ev_main = nullptr;
     // Blocks per SM given to the dA/dt kernel while another block's solve may run beside it.
     int overlap_blocks_per_sm = 2;
     // The coil field table (cunibs_context_set_coil_table): mode 1 reads it for nodes deeper than
     // table_near_m below the coil, mode 0 sums every dipole at every node.
     CoilTable coil_table;
+    // The host coil the table was last built for (positions, then moments); empty when it came from device memory.
+    std::vector<double> table_coil;
     int table_mode = 1;
     double table_near_m = 0.015, table_step = 0.035;
     double mesh_rho_m = 0.0;  // largest distance of a node from the centre of the mesh's bounding box
@@ -202,14 +219,10 @@ struct cunibs_context {
     ~cunibs_context() {
         for (cudaEvent_t e : ev)
             if (e) cudaEventDestroy(e);
-        for (BlockSlot& sl : slots) {
+        for (BlockSlot& sl : slots)
             if (sl.prepared) cudaEventDestroy(sl.prepared);
-            if (sl.h_deg) cudaFreeHost(sl.h_deg);
-            if (sl.h_near) cudaFreeHost(sl.h_near);
-        }
         if (ev_main) cudaEventDestroy(ev_main);
-        if (h_coil_flag) cudaFreeHost(h_coil_flag);
-        if (staging) cudaFreeHost(staging);
+        if (pinned) cudaFreeHost(pinned);
         solver.reset();
         if (prep) cudaStreamDestroy(prep);
         if (stream) cudaStreamDestroy(stream);
@@ -240,6 +253,7 @@ Params resolve(const cunibs_context* c, const cunibs_solve_opts* o) {
 }
 
 constexpr int kMaxBlock = 16;
+static_assert(sizeof(Pinned::deg) == 2 * kMaxBlock * sizeof(int), "one flag per placement of a block");
 // Eigenvalues of a placement's Jacobi-scaled sensitivity Gram kept for its draw guesses, relative
 // to the largest (the reference keeps singular values above 1e-8 of the largest, run.py:108-123).
 constexpr double kSigmaRtol = 1e-12;
@@ -289,35 +303,72 @@ long long prepare_block(cunibs_context* c, const double* pos, const double* mom,
         if (timed) c->mark(i, ps);
     };
     const int n_red = m.n_nodes - 1;
+    // The coil's kind (all moments along its own z axis, or not) picks the dA/dt kernel, and the table
+    // follows the coil. Host inputs are looked at here, while they are on the host; a device coil takes two
+    // kernels and a wait.
+    CoilTable& tb = c->coil_table;
+    const bool want_table = c->table_mode != 0;
+    const std::size_t n3 = 3 * static_cast<std::size_t>(n_dip), k3 = 3 * static_cast<std::size_t>(k);
+    bool general = false, other_coil = false, coil_known = false;
+    const double *host_pos = nullptr, *host_mom = nullptr;
     if (host_inputs) {
-        sl.in_pos.upload(pos, 3 * static_cast<std::size_t>(n_dip), ps);
-        sl.in_mom.upload(mom, 3 * static_cast<std::size_t>(n_dip), ps);
-        sl.in_centers.upload(centers, 3 * static_cast<std::size_t>(k), ps);
-        if (handles) sl.in_handles.upload(handles, 3 * static_cast<std::size_t>(k), ps);
-        sl.in_dists.upload(dists, static_cast<std::size_t>(k), ps);
-        pos = sl.in_pos.get();
-        mom = sl.in_mom.get();
-        centers = sl.in_centers.get();
-        handles = handles ? sl.in_handles.get() : nullptr;
-        dists = sl.in_dists.get();
+        host_pos = pos;
+        host_mom = mom;
+        for (std::size_t j = 0; j < n3; j += 3) general = general || mom[j] != 0.0 || mom[j + 1] != 0.0;
+        coil_known = !tb.built || tb.n_dip != n_dip || c->table_coil.size() == 2 * n3;
+        if (c->table_coil.size() == 2 * n3)
+            other_coil = std::memcmp(c->table_coil.data(), pos, n3 * sizeof(double)) != 0 ||
+                         std::memcmp(c->table_coil.data() + n3, mom, n3 * sizeof(double)) != 0;
+        // The coil of the table in use is on the device already.
+        const bool on_device = tb.built && c->table_coil.size() == 2 * n3 && !other_coil && want_table &&
+                               tb.near_m == c->table_near_m && tb.step == c->table_step;
+        const double* parts[5] = {pos, mom, centers, handles, dists};
+        const std::size_t lens[5] = {on_device ? 0 : n3, on_device ? 0 : n3, k3, handles ? k3 : 0,
+                                     static_cast<std::size_t>(k)};
+        sl.in.reserve(2 * n3 + 7 * kMaxBlock);
+        const double* dev[5];
+        std::size_t at = 0;
+        const bool staged = on_device || n_dip <= kPinnedDipoles;
+        // The slot's last block may have been cancelled with its copy still in flight.
+        if (staged) CUNIBS_CHECK(cudaEventSynchronize(sl.prepared));
+        for (int i = 0; i < 5; ++i) {
+            dev[i] = sl.in.get() + at;
+            if (lens[i] != 0) {
+                if (staged) std::memcpy(sl.h_in + at, parts[i], lens[i] * sizeof(double));
+                else CUNIBS_CHECK(cudaMemcpyAsync(sl.in.get() + at, parts[i], lens[i] * sizeof(double), cudaMemcpyHostToDevice, ps));
+            }
+            at += lens[i];
+        }
+        if (staged) CUNIBS_CHECK(cudaMemcpyAsync(sl.in.get(), sl.h_in, at * sizeof(double), cudaMemcpyHostToDevice, ps));
+        else CUNIBS_CHECK(cudaStreamSynchronize(ps));  // the caller's memory may be pinned, and is the caller's again
+        pos = on_device ? tb.pos.get() : dev[0];
+        mom = on_device ? tb.mom.get() : dev[1];
+        centers = dev[2];
+        handles = handles ? dev[3] : nullptr;
+        dists = dev[4];
     }
-    // The coil's kind (all moments along its own z axis, or not) picks the dA/dt kernel.
     c->zdip_packed.reserve(packed_zdipole_bytes() * static_cast<std::size_t>(n_dip));
     c->coil_flag.reserve(1);
     prep_zdipoles(pos, mom, n_dip, c->zdip_packed.get(), c->coil_flag.get(), ps);
-    CoilTable& tb = c->coil_table;
-    const bool want_table = c->table_mode != 0;
-    if (want_table && tb.built && tb.n_dip == n_dip) coil_compare(pos, mom, n_dip, tb, c->coil_flag.get(), ps);
-    CUNIBS_CHECK(cudaMemcpyAsync(c->h_coil_flag, c->coil_flag.get(), sizeof(int), cudaMemcpyDeviceToHost, ps));
-    CUNIBS_CHECK(cudaStreamSynchronize(ps));
-    const bool zcoil = (*c->h_coil_flag & 1) == 0;
-    // The table follows the coil: rebuilt (once) when the coil, its kind or the table's parameters
-    // change.
-    if (want_table && (!tb.built || tb.n_dip != n_dip || (*c->h_coil_flag & 2) || tb.nc != (zcoil ? 2 : 3) ||
+    if (!coil_known) {
+        if (want_table && tb.built && tb.n_dip == n_dip) coil_compare(pos, mom, n_dip, tb, c->coil_flag.get(), ps);
+        CUNIBS_CHECK(cudaMemcpyAsync(c->h_coil_flag, c->coil_flag.get(), sizeof(int), cudaMemcpyDeviceToHost, ps));
+        CUNIBS_CHECK(cudaStreamSynchronize(ps));
+        general = (*c->h_coil_flag & 1) != 0;
+        other_coil = (*c->h_coil_flag & 2) != 0;
+    }
+    const bool zcoil = !general;
+    // The table is rebuilt (once) when the coil, its kind or the table's parameters change.
+    if (want_table && (!tb.built || tb.n_dip != n_dip || other_coil || tb.nc != (zcoil ? 2 : 3) ||
                        tb.near_m != c->table_near_m || tb.step != c->table_step)) {
         const double rho = std::max(c->mesh_rho_m, c->table_near_m);
+        c->table_coil.clear();
         build_coil_table(tb, pos, mom, n_dip, zcoil, c->zdip_packed.get(), c->table_near_m, c->table_step, 1.1 * rho,
                          2.5 * rho + 0.05, kCoilTableMaxPoints, ps);
+        if (host_inputs) {
+            c->table_coil.assign(host_pos, host_pos + n3);
+            c->table_coil.insert(c->table_coil.end(), host_mom, host_mom + n3);
+        }
     }
     const bool use_table = want_table && tb.valid;
     // The slot's previous block is finished on the context stream: start after what that stream
@@ -522,8 +573,9 @@ void block_outputs_host(cunibs_context* c, const PendingBlock& pb, const SolveSt
     cudaStream_t s = c->stream;
     const int k = pb.k;
     const cunibs_solve_opts* opts = pb.has_opts ? &pb.opts : nullptr;
-    copy_out(out->transforms, c->slots[pb.slot].T.get(), sizeof(double) * 16 * k, cudaMemcpyDeviceToHost, s);
-    copy_out(out->summary, c->summary.get(), sizeof(double) * kSummaryLen * k, cudaMemcpyDeviceToHost, s);
+    // The small outputs through pinned memory: nothing waits on a pageable copy of theirs.
+    copy_out(c->pinned->transforms, c->slots[pb.slot].T.get(), sizeof(double) * 16 * k, cudaMemcpyDeviceToHost, s);
+    copy_out(c->pinned->summary, c->summary.get(), sizeof(double) * kSummaryLen * k, cudaMemcpyDeviceToHost, s);
     copy_out(out->magnE, c->magn.get(), sizeof(float) * static_cast<std::size_t>(m.n_tets) * k, cudaMemcpyDeviceToHost, s);
     copy_out(out->E, c->E.get(), sizeof(float) * 3 * static_cast<std::size_t>(m.n_tets) * k, cudaMemcpyDeviceToHost, s);
     copy_out(out->E_slots, c->e_slots.get(), slot_bytes(c, opts, k), cudaMemcpyDeviceToHost, s);
@@ -533,6 +585,8 @@ void block_outputs_host(cunibs_context* c, const PendingBlock& pb, const SolveSt
         copy_out(out->v, c->v.get(), sizeof(double) * static_cast<std::size_t>(m.n_nodes) * k, cudaMemcpyDeviceToHost, s);
     }
     CUNIBS_CHECK(cudaStreamSynchronize(s));
+    std::memcpy(out->transforms, c->pinned->transforms, sizeof(double) * 16 * k);
+    std::memcpy(out->summary, c->pinned->summary, sizeof(double) * kSummaryLen * k);
     for (int i = 0; i < k; ++i) {
         if (out->iterations) out->iterations[i] = st.col_iters[i];
         if (out->relres) out->relres[i] = st.col_rel[i];
@@ -646,14 +700,15 @@ int cunibs_context_create(const double* nodes_mm, int n_nodes, const int* tet_no
         CUNIBS_CHECK(cudaStreamCreateWithPriority(&c->prep, cudaStreamNonBlocking, least));
         CUNIBS_CHECK(cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device));
         CUNIBS_CHECK(cudaEventCreateWithFlags(&c->ev_main, cudaEventDisableTiming));
-        CUNIBS_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&c->h_coil_flag), sizeof(int), cudaHostAllocDefault));
-        CUNIBS_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&c->staging), sizeof(Staging), cudaHostAllocDefault));
-        for (BlockSlot& sl : c->slots) {
+        CUNIBS_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&c->pinned), sizeof(Pinned), cudaHostAllocDefault));
+        c->h_coil_flag = &c->pinned->coil_flag;
+        c->staging = &c->pinned->staging;
+        for (int i = 0; i < 2; ++i) {
+            BlockSlot& sl = c->slots[i];
             CUNIBS_CHECK(cudaEventCreateWithFlags(&sl.prepared, cudaEventDisableTiming));
-            CUNIBS_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&sl.h_deg), sizeof(int) * kMaxBlock,
-                                       cudaHostAllocDefault));
-            CUNIBS_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&sl.h_near), sizeof(int) * kMaxBlock,
-                                       cudaHostAllocDefault));
+            sl.h_deg = c->pinned->deg[i];
+            sl.h_near = c->pinned->near[i];
+            sl.h_in = c->pinned->in[i];
         }
         {
             double lo[3] = {nodes_mm[0], nodes_mm[1], nodes_mm[2]}, hi[3] = {lo[0], lo[1], lo[2]};

@@ -1312,7 +1312,7 @@ class Solver {
     DevArray<double> tolv;
     DevArray<int> frozen, outer_conv, conv_iter, iter_counter;
     DevArray<unsigned> counter;
-    int* h_flags = nullptr;   // pinned
+    int* h_flags = nullptr;   // pinned, behind h_dbl
     double* h_dbl = nullptr;  // pinned
     // Deferred readbacks of the last solve_plain: h_dbl[2K..3K) holds the right-hand side norms
     // (check_ref), h_flags[2K] the device loop's iteration count (st.iterations == -1).
@@ -1322,7 +1322,6 @@ class Solver {
 
     ~Solver() {
         for (auto& kv : graphs) cudaGraphExecDestroy(kv.second.first);
-        if (h_flags) cudaFreeHost(h_flags);
         if (h_dbl) cudaFreeHost(h_dbl);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -1366,10 +1365,11 @@ class Solver {
         counter.resize(1);
         counter.zero(stream);
         partials.resize(static_cast<std::size_t>(kMaxReduceBlocks) * K);
-        if (h_flags) cudaFreeHost(h_flags);
-        if (h_dbl) cudaFreeHost(h_dbl);
-        CUNIBS_CHECK(cudaMallocHost(&h_flags, sizeof(int) * 4 * K));
-        CUNIBS_CHECK(cudaMallocHost(&h_dbl, sizeof(double) * 4 * K));
+        if (!h_dbl) {  // one allocation for the widest block
+            constexpr int kWidest = 16;
+            CUNIBS_CHECK(cudaMallocHost(&h_dbl, (sizeof(double) + sizeof(int)) * 4 * kWidest));
+            h_flags = reinterpret_cast<int*>(h_dbl + 4 * kWidest);
+        }
         kcap = K;
         CUNIBS_CHECK(cudaStreamSynchronize(stream));
     }

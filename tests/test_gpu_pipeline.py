@@ -12,6 +12,7 @@ import pytest
 import torch
 
 from cunibs_b200 import Placement, Subject, _native
+from cunibs_b200.coil import Coil
 from cunibs_b200.synthetic import figure8_coil, sphere_head
 
 pytestmark = pytest.mark.gpu
@@ -158,3 +159,29 @@ def test_iter_simulate_pipelines_and_cleans_up(sphere_ctx):
     gen.close()
     assert subj.context.pending == 0
     subj.free()
+
+
+@pytest.mark.parametrize("n_per_wing", [1, 2048, 2049])
+def test_host_inputs_are_the_callers_again_after_submit(sphere_ctx, n_per_wing):
+    """2, 4096 and 4098 dipoles (up to 4096 go through pinned memory): a coil and placements overwritten
+    right after each submit, pinned or not, a new coil in every other block."""
+    m, ctx = sphere_ctx
+    coils = [figure8_coil(n_per_wing), figure8_coil(n_per_wing, disc_radius_mm=30.0)]
+    blocks = _blocks(4, seed=7)
+    fresh = _native.Context(m.nodes_mm, m.tet_nodes, m.tet_tags, m.skin_tris)
+    want = [fresh.solve_block(coils[b // 2], *blocks[b], 1e6, **KW) for b in range(4)]
+    fresh.close()
+    for pinned in (False, True):
+        own = (lambda a: torch.from_numpy(a.copy()).pin_memory().numpy()) if pinned else np.copy
+        tickets, got = [], []
+        for b in range(4):
+            pos, mom = own(coils[b // 2].positions_m), own(coils[b // 2].moments)
+            c, h, d = (own(a) for a in blocks[b])
+            tickets.append(ctx.submit_block(Coil(positions_m=pos, moments=mom, name="own"), c, h, d, 1e6, **KW))
+            for a in (pos, mom, c, h, d):
+                a[:] = 1.0
+            if len(tickets) == 2:
+                got.append(ctx.finish_block(tickets.pop(0)))
+        got.append(ctx.finish_block(tickets.pop(0)))
+        for a, b in zip(got, want):
+            _same(a, b)
