@@ -166,6 +166,8 @@ def load() -> C.CDLL:
         "cunibs_adm_evaluate_exact": ([_vp, dp, dp, C.c_int, dp, C.c_int, C.c_double, dp, dp], C.c_int),
         "cunibs_context_array": ([_vp, C.c_char_p, C.c_int, _vp, C.c_longlong, C.POINTER(C.c_longlong)], C.c_int),
         "cunibs_context_place": ([_vp, _vp, _vp, _vp, C.c_int, _vp, _vp], C.c_int),
+        "cunibs_context_select": ([_vp, C.c_int, _vp, C.c_double, C.POINTER(C.c_int)], C.c_int),
+        "cunibs_context_selected": ([_vp, _vp, _vp, C.c_int], C.c_int),
         "cunibs_context_dadt": ([_vp, _vp, _vp, C.c_int, _vp, C.c_int, C.c_double, _vp], C.c_int),
         "cunibs_context_solve": ([_vp, _vp, _vp, C.c_int, C.c_int, C.c_int, C.c_double, C.c_int, _vp, _vp, _vp], C.c_int),
         "cunibs_context_vcycle": ([_vp, _vp, _vp, C.c_int, C.c_int], C.c_int),
@@ -337,6 +339,18 @@ class Context:
         deg = np.empty(k, np.int32)
         check(self._lib.cunibs_context_place(self.handle, _p(centers), _p(handles_a), _p(dists), k, _p(T), _p(deg)))
         return T, deg
+
+    def select_elements(self, tag: int, position_mm, radius_mm: float):
+        """cunibs_context_select: (indices, barycentres (n, 3) mm, volumes (n)) of a target's elements;
+        empty when the mesh has no element of the tissue."""
+        p = np.ascontiguousarray(position_mm, np.float64).reshape(3)
+        n = C.c_int(0)
+        check(self._lib.cunibs_context_select(self.handle, int(tag), _p(p), float(radius_mm), C.byref(n)))
+        idx = np.empty(n.value, np.int32)
+        rec = np.empty((n.value, 4))
+        if n.value:
+            check(self._lib.cunibs_context_selected(self.handle, _p(idx), _p(rec), n.value))
+        return idx, np.ascontiguousarray(rec[:, :3]), np.ascontiguousarray(rec[:, 3])
 
     def dadt(self, coil, transforms, didt) -> np.ndarray:
         T = np.ascontiguousarray(transforms, np.float64).reshape(-1, 16)

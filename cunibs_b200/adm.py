@@ -80,28 +80,20 @@ class ResolvedTarget:
 def resolve_target(subject, target: Target) -> ResolvedTarget:
     """Map a :class:`Target` to region elements, volume weights and directions (target.py:75-109)."""
     ctx = _context(subject)
-    barys = ctx.array("bary").reshape(-1, 3)
-    tags = ctx.array("tet_tags")
-    vols = ctx.array("vols")
-    region_ids = np.flatnonzero(metrics.region_mask(tags, target.region)).astype(np.int32)
-    if region_ids.size == 0:
+    tag = -1 if target.region == "all" else metrics.region_tag(target.region)
+    # On the GPU: the mesh's barycentres, tags and volumes stay there.
+    sel, barys, vols = ctx.select_elements(tag, target.position_mm, target.radius_mm)
+    if sel.size == 0:
         raise ValueError(f"Region {target.region!r} contains no elements.")
-    d2 = ((barys[region_ids] - target.position_mm) ** 2).sum(1)
-    if target.radius_mm <= 0.0:
-        sel = region_ids[[int(np.argmin(d2))]]
-    else:
-        within = d2 <= target.radius_mm ** 2
-        if not within.any():
-            within = d2 == d2.min()
-        sel = region_ids[within]
-    v = vols[sel].astype(np.float64)
-    weights = v / v.sum()
+    if target.radius_mm > 0.0 and np.isnan(target.position_mm).any():
+        sel, barys, vols = sel[:0], barys[:0], vols[:0]  # nothing is near, or nearest to, a point that is none
+    weights = vols / vols.sum()
     if target.direction is None:
         directions, magnitude = np.eye(3), True
     else:
         directions, magnitude = np.asarray(target.direction, np.float64)[None], False
-    return ResolvedTarget(elem_idx=np.ascontiguousarray(sel), weights=weights, directions=directions,
-                          magnitude=magnitude, barycenter_mm=weights @ barys[sel])
+    return ResolvedTarget(elem_idx=sel, weights=weights, directions=directions, magnitude=magnitude,
+                          barycenter_mm=weights @ barys)
 
 
 # --- grid (grid.py) ----------------------------------------------------------------------------

@@ -10,6 +10,7 @@
 //     Q_d(g) = mu0/4pi sum_n W_n x (g - r_n) / |g - r_n|^3
 // then gives E_d = didt sum_j m_j . Q_d(s_j) for the placed coil dipoles (s_j, m_j).
 #include <algorithm>
+#include <cub/cub.cuh>
 #include <climits>
 #include <cmath>
 
@@ -17,6 +18,70 @@
 
 namespace cunibs {
 namespace {
+
+// Squared distance (mm^2) of an element's barycentre from a point, every product and sum rounded on its own in the order
+// of the axes, as an array language's ((b - p) ** 2).sum(1) rounds them.
+__device__ __forceinline__ double bary_d2(const double* __restrict__ bary, int e, double px, double py, double pz) {
+    const double dx = bary[3 * static_cast<long>(e)] - px, dy = bary[3 * static_cast<long>(e) + 1] - py;
+    const double dz = bary[3 * static_cast<long>(e) + 2] - pz;
+    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+}
+
+// Elements of tissue `tag` (every element when tag < 0): flags[e] = d2 <= limit, *nearest = the bits of the smallest d2
+// (non-negative, so the bits order as the values), *members = their number.
+__global__ void __launch_bounds__(kBlock) select_near_kernel(const double* __restrict__ bary,
+                                                             const int* __restrict__ tags, int n, int tag, double px,
+                                                             double py, double pz, double limit,
+                                                             int* __restrict__ flags,
+                                                             unsigned long long* __restrict__ nearest,
+                                                             int* __restrict__ members) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long bits = ~0ull;
+    int in = 0;
+    if (e < n) {
+        in = tag < 0 || tags[e] == tag;
+        const double d2 = in ? bary_d2(bary, e, px, py, pz) : 0.0;
+        flags[e] = in && d2 <= limit;
+        if (in) bits = static_cast<unsigned long long>(__double_as_longlong(d2));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, bits, o);
+        bits = v < bits ? v : bits;
+    }
+    const unsigned any = __ballot_sync(0xffffffffu, in);
+    if ((threadIdx.x & 31) == 0 && any != 0) {
+        atomicMin(nearest, bits);
+        atomicAdd(members, __popc(any));
+    }
+}
+
+// flags[e] = the element is of the tissue and as near as the nearest.
+__global__ void select_nearest_kernel(const double* __restrict__ bary, const int* __restrict__ tags, int n, int tag,
+                                      double px, double py, double pz, const unsigned long long* __restrict__ nearest,
+                                      int* __restrict__ flags) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    flags[e] = (tag < 0 || tags[e] == tag) &&
+               static_cast<unsigned long long>(__double_as_longlong(bary_d2(bary, e, px, py, pz))) == *nearest;
+}
+
+// The flagged elements in order: index, barycentre and volume.
+__global__ void select_compact_kernel(const int* __restrict__ flags, const int* __restrict__ pos, int n,
+                                      const double* __restrict__ bary, const double* __restrict__ vols,
+                                      int* __restrict__ idx, double* __restrict__ out) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n || !flags[e]) return;
+    const long q = pos[e];
+    idx[q] = e;
+    for (int a = 0; a < 3; ++a) out[4 * q + a] = bary[3 * static_cast<long>(e) + a];
+    out[4 * q + 3] = vols[e];
+}
+
+__global__ void scatter_weights_kernel(const int* __restrict__ idx, const double* __restrict__ weights, int n,
+                                       double* __restrict__ alpha) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) alpha[idx[i]] = weights[i];
+}
 
 // c_red[r][d] = sum over the corners of node i of alpha_e (dir_d . g_corner), FP64, node-to-corner
 // order; columns past n_dir repeat the last direction.
@@ -223,6 +288,56 @@ __global__ void __launch_bounds__(kEvalThreads) exact_reduce_kernel(const float*
 }
 
 }  // namespace
+
+int adm_select(const Mesh& m, int tag, const double* p, double radius_mm, AdmSelection& sel, cudaStream_t s) {
+    const int n = m.n_tets;
+    sel.count = 0;
+    sel.flags.reserve(static_cast<std::size_t>(n) + 1);
+    sel.pos.reserve(static_cast<std::size_t>(n) + 1);
+    sel.nearest.reserve(1);
+    sel.members.reserve(1);
+    sel.members.zero(s);
+    CUNIBS_CHECK(cudaMemsetAsync(sel.nearest.get(), 0xFF, sizeof(unsigned long long), s));
+    CUNIBS_CHECK(cudaMemsetAsync(sel.flags.get() + n, 0, sizeof(int), s));
+    select_near_kernel<<<grid_for(n), kBlock, 0, s>>>(m.bary.get(), m.tags.get(), n, tag, p[0], p[1], p[2],
+                                                      radius_mm > 0.0 ? radius_mm * radius_mm : -1.0, sel.flags.get(),
+                                                      sel.nearest.get(), sel.members.get());
+    count_launch();
+    auto count = [&] {
+        std::size_t bytes = 0;
+        CUNIBS_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, sel.flags.get(), sel.pos.get(), n + 1, s));
+        sel.temp.reserve(bytes);
+        CUNIBS_CHECK(cub::DeviceScan::ExclusiveSum(sel.temp.get(), bytes, sel.flags.get(), sel.pos.get(), n + 1, s));
+        int total = 0, members = 0;
+        CUNIBS_CHECK(cudaMemcpyAsync(&total, sel.pos.get() + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CUNIBS_CHECK(cudaMemcpyAsync(&members, sel.members.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+        CUNIBS_CHECK(cudaStreamSynchronize(s));
+        return members == 0 ? -1 : total;
+    };
+    int found = count();
+    if (found < 0) return 0;
+    if (found == 0) {
+        select_nearest_kernel<<<grid_for(n), kBlock, 0, s>>>(m.bary.get(), m.tags.get(), n, tag, p[0], p[1], p[2],
+                                                             sel.nearest.get(), sel.flags.get());
+        count_launch();
+        found = count();
+    }
+    sel.idx.reserve(found);
+    sel.data.reserve(4 * static_cast<std::size_t>(found));
+    select_compact_kernel<<<grid_for(n), kBlock, 0, s>>>(sel.flags.get(), sel.pos.get(), n, m.bary.get(), m.vols.get(),
+                                                         sel.idx.get(), sel.data.get());
+    count_launch();
+    CUNIBS_LAUNCH_CHECK("element selection");
+    sel.count = radius_mm <= 0.0 ? 1 : found;  // no radius: the first of the nearest
+    return sel.count;
+}
+
+void adm_scatter_weights(const int* idx, const double* weights, int n, DevArray<double>& alpha, cudaStream_t s) {
+    alpha.zero(s);
+    scatter_weights_kernel<<<grid_for(n), kBlock, 0, s>>>(idx, weights, n, alpha.get());
+    count_launch();
+    CUNIBS_LAUNCH_CHECK("adm target weights");
+}
 
 void adm_adjoint_rhs(const Mesh& m, const double* alpha, const AdmDirections& dirs, int K, double* c_red,
                      cudaStream_t s) {

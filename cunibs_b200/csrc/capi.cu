@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
+#include <map>
 #include <string>
 #include <type_traits>
 
@@ -169,6 +170,8 @@ struct cunibs_context {
     std::unique_ptr<WarmStart> warm;
     std::vector<int> warm_used;
     std::vector<double> init_rel;
+    // The last element selection (cunibs_context_select).
+    AdmSelection selection;
     // The open conductivity study, if any (its block slot is reserved while it is open).
     std::unique_ptr<SigmaStudy> study;
     // Stage timing (CUDA events on the context stream), enabled by cunibs_context_set_timing.
@@ -1275,6 +1278,27 @@ void adm_inputs(cunibs_adm* a, const double* dip_pos_m, const double* dip_moment
 
 extern "C" {
 
+int cunibs_context_select(cunibs_context* c, int tag, const double* position_mm, double radius_mm, int* count) {
+    return guarded([&] {
+        require(c && position_mm && count, "NULL argument");
+        require(tag >= -1 && tag <= 10, "tag must be a tissue tag in [0, 10], or -1 for every element");
+        DeviceGuard dg(c->device);
+        *count = adm_select(c->mesh, tag, position_mm, radius_mm, c->selection, c->stream);
+    });
+}
+
+int cunibs_context_selected(const cunibs_context* c, int* elem_idx, double* bary_vol, int cap) {
+    return guarded([&] {
+        require(c && elem_idx && bary_vol, "NULL argument");
+        require(cap >= c->selection.count, "output buffers too small");
+        DeviceGuard dg(c->device);
+        const std::size_t n = c->selection.count;
+        c->selection.idx.download(elem_idx, n, c->stream);
+        c->selection.data.download(bary_vol, 4 * n, c->stream);
+        CUNIBS_CHECK(cudaStreamSynchronize(c->stream));
+    });
+}
+
 int cunibs_adm_create(cunibs_context* c, const int* elem_idx, const double* weights, int n_elem,
                       const double* directions, int n_dir, double tolerance, int max_iters, int* iterations,
                       double* relres, cunibs_adm** out) {
@@ -1287,11 +1311,17 @@ int cunibs_adm_create(cunibs_context* c, const int* elem_idx, const double* weig
         require(!c->study, "a conductivity study is open: end it first");
         require(c->pending.empty(), "finish the submitted blocks first");
         Mesh& m = c->mesh;
-        std::vector<double> alpha(m.n_tets, 0.0);
+        std::map<int, double> target;  // an element named twice has both weights
         for (int i = 0; i < n_elem; ++i) {
             require(elem_idx[i] >= 0 && elem_idx[i] < m.n_tets, "target element index out of range");
             require(std::isfinite(weights[i]), "target weights must be finite");
-            alpha[elem_idx[i]] += weights[i];
+            target[elem_idx[i]] += weights[i];
+        }
+        std::vector<int> t_idx;
+        std::vector<double> t_w;
+        for (const auto& t : target) {
+            t_idx.push_back(t.first);
+            t_w.push_back(t.second);
         }
         auto a = std::make_unique<cunibs_adm>();
         a->ctx = c;
@@ -1306,7 +1336,12 @@ int cunibs_adm_create(cunibs_context* c, const int* elem_idx, const double* weig
         }
         DeviceGuard dg(c->device);
         cudaStream_t s = c->stream;
-        a->alpha.upload(alpha.data(), alpha.size(), s);
+        DevArray<int> d_idx;
+        DevArray<double> d_w;
+        d_idx.upload(t_idx.data(), t_idx.size(), s);
+        d_w.upload(t_w.data(), t_w.size(), s);
+        a->alpha.resize(m.n_tets);
+        adm_scatter_weights(d_idx.get(), d_w.get(), static_cast<int>(t_idx.size()), a->alpha, s);
         const int K = n_dir == 1 ? 1 : (n_dir == 2 ? 2 : 4);
         const int n_red = m.n_nodes - 1;
         DevArray<double> B(static_cast<std::size_t>(n_red) * K), X(static_cast<std::size_t>(n_red) * K);

@@ -455,6 +455,19 @@ struct AdmGrid {
     double spacing_mm[3];
     int shape[3];
 };
+// A target's elements: those of tissue `tag` (any when < 0) whose barycentre lies within radius_mm of p, the nearest ones where
+// none does, the first of the nearest where radius_mm <= 0. Returns their number (0 when the mesh has no
+// element of the tissue); sel keeps their indices, ascending, and {barycentre, volume} records.
+struct AdmSelection {
+    DevArray<int> flags, pos, members, idx;
+    DevArray<unsigned long long> nearest;
+    DevArray<unsigned char> temp;
+    DevArray<double> data;
+    int count = 0;
+};
+int adm_select(const Mesh& m, int tag, const double* p, double radius_mm, AdmSelection& sel, cudaStream_t s);
+// alpha = weights at idx (n of them, distinct), zero elsewhere.
+void adm_scatter_weights(const int* idx, const double* weights, int n, DevArray<double>& alpha, cudaStream_t s);
 // Adjoint right-hand sides (n_red, K) of the target weights alpha (per element, zero off target).
 void adm_adjoint_rhs(const Mesh& m, const double* alpha, const AdmDirections& dirs, int K, double* c_red,
                      cudaStream_t s);

@@ -281,6 +281,14 @@ int cunibs_sigma_coefficients(int n_tags, const double* gram, const double* proj
 
 typedef struct cunibs_adm cunibs_adm;
 
+/* A target's elements (adm/target.py:75-109): those of tissue `tag` (every element when -1) whose barycentre lies within
+ * radius_mm of position_mm; where none does, the nearest (all at its distance); with radius_mm <= 0 the
+ * first of the nearest. *count receives their number, 0 when the mesh has no element of the tissue. The
+ * selection is kept until the next one; cunibs_context_selected copies it to host buffers of at least that many:
+ * indices, ascending, and (count, 4) records of barycentre (mm) and volume (m^3). */
+int cunibs_context_select(cunibs_context* ctx, int tag, const double* position_mm, double radius_mm, int* count);
+int cunibs_context_selected(const cunibs_context* ctx, int* elem_idx, double* bary_vol, int cap);
+
 /* The adjoint (reciprocity) solves of a target functional J_d = sum_i weights[i] (dir_d . E_e),
  * e = elem_idx[i] in the context's element order, for n_dir (1..3) directions (replaces
  * solve_adjoint, reciprocity.py:119-141): K lambda_d = c_d, all directions in one block solve to
