@@ -155,19 +155,6 @@ __global__ void centred_nodes_kernel(const double* __restrict__ nodes_mm, int n,
     out_m[3 * static_cast<long>(i) + 2] = (nodes_mm[3 * static_cast<long>(i) + 2] - cz) * 1e-3;
 }
 
-// Grid points in C order (x slowest), mm.
-__global__ void grid_points_kernel(AdmGrid gr, double* __restrict__ out) {
-    const long q = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const long total = static_cast<long>(gr.shape[0]) * gr.shape[1] * gr.shape[2];
-    if (q >= total) return;
-    const int iz = static_cast<int>(q % gr.shape[2]);
-    const int iy = static_cast<int>((q / gr.shape[2]) % gr.shape[1]);
-    const int ix = static_cast<int>(q / (static_cast<long>(gr.shape[1]) * gr.shape[2]));
-    out[3 * q] = gr.origin_mm[0] + gr.spacing_mm[0] * ix;
-    out[3 * q + 1] = gr.origin_mm[1] + gr.spacing_mm[1] * iy;
-    out[3 * q + 2] = gr.origin_mm[2] + gr.spacing_mm[2] * iz;
-}
-
 constexpr int kEvalThreads = 256;
 constexpr double kIndexTol = 1e-6;  // slack on the fractional grid index (3 nm at 3 mm)
 
@@ -369,12 +356,6 @@ void adm_centred_nodes(const Mesh& m, const double* center_mm, double* out_m, cu
     centred_nodes_kernel<<<grid_for(m.n_nodes), kBlock, 0, s>>>(m.nodes.get(), m.n_nodes, center_mm[0], center_mm[1],
                                                                center_mm[2], out_m); count_launch();
     CUNIBS_LAUNCH_CHECK("adm centred nodes");
-}
-
-void adm_grid_points(const AdmGrid& gr, double* out, cudaStream_t s) {
-    const long total = static_cast<long>(gr.shape[0]) * gr.shape[1] * gr.shape[2];
-    grid_points_kernel<<<grid_for(total), kBlock, 0, s>>>(gr, out); count_launch();
-    CUNIBS_LAUNCH_CHECK("adm grid points");
 }
 
 void adm_evaluate(const float* Q, int n_dir, const AdmGrid& gr, const double* pos, const double* mom, int n_dip,

@@ -1225,12 +1225,11 @@ struct cunibs_adm {
     AdmGrid grid{};
     DevArray<float> Q;               // (n_dir, n_grid, 3)
     DevArray<double> pos, mom, T, E; // evaluation workspace
-    // Sampling workspace, grown on demand and kept, so that a repeated sampling allocates nothing:
-    // the grid points, the sources' centred positions, their packed records and frames, and the
-    // per-chunk partial fields.
-    DevArray<double> q_pts, q_src, q_T;
-    DevArray<unsigned char> q_packed;
+    // Sampling workspace, grown on demand and kept, so that a repeated sampling allocates nothing: the
+    // sources, and their runs' partial fields.
     DevArray<float> q_part;
+    DevArray<double> q_sources;
+    DevArray<double> q_src;  // the sources' centred positions (evaluation at the dipoles themselves)
     DevArray<unsigned long long> bad;
 };
 
@@ -1416,22 +1415,11 @@ int cunibs_adm_sample(cunibs_adm* a, const double* origin_mm, const double* spac
         require(n_grid <= (1LL << 28), "at most 2^28 grid points");
         DeviceGuard dg(a->ctx->device);
         cudaStream_t s = a->ctx->stream;
-        double center[3];
-        for (int x = 0; x < 3; ++x) center[x] = gr.origin_mm[x] + 0.5 * gr.spacing_mm[x] * (gr.shape[x] - 1);
-        DevArray<double>& pts = a->q_pts;
-        DevArray<double>& Td = a->q_T;
-        DevArray<unsigned char>& packed = a->q_packed;
-        pts.reserve(3 * static_cast<std::size_t>(n_grid));
-        adm_grid_points(gr, pts.get(), s);
-        adm_sources(a, center, packed, Td, s);
         a->sampled = false;
         a->Q.resize(3 * static_cast<std::size_t>(n_grid) * a->dirs.n);
-        // Q_d on the grid: the coil-field N-body with the mesh nodes as sources (reciprocity.py:183-213),
-        // every direction in one pass over the sources.
-        dadt_nodes_shared(pts.get(), static_cast<int>(n_grid), reinterpret_cast<const float*>(packed.get()),
-                          a->ctx->mesh.n_nodes, Td.get(), a->dirs.n, 1.0, a->Q.get(), s, a->q_part);
-        CUNIBS_LAUNCH_CHECK("reciprocity field");
-        CUNIBS_CHECK(cudaStreamSynchronize(s));
+        // Q_d on the grid: the coil-field N-body with the mesh nodes as sources (reciprocity.py:183-213).
+        qfield_sample(a->ctx->mesh, gr, a->W.get(), a->dirs.n, a->Q.get(), a->q_sources, a->q_part,
+                      a->ctx->sm_count, s);
         a->grid = gr;
         a->sampled = true;
     });

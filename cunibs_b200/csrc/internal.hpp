@@ -208,14 +208,6 @@ void dadt_elements(const Mesh& m, const float* dadt_nodes, int k, float* dadt_el
 // The general-moment dA/dt on raw device node coordinates (no Mesh), packed records from prep_dipoles.
 void dadt_nodes_raw(const double* nodes_mm, int n_nodes, const float* dip_packed, int n_dip,
                     const double* transforms_dev, int k, double didt, float* out, cudaStream_t s);
-// n_sets (1..3) source sets at common positions, records set * n_dip + j of prep_dipoles all made
-// with the one transform transform_dev; out (n_sets, n_nodes, 3). Set d's field is bitwise
-// dadt_nodes_raw's for that set alone; each pair's geometry is formed once for all sets.
-// scratch holds the source chunks' partial fields when the targets alone do not fill the GPU (grown
-// on demand and kept by the caller, so repeated calls allocate nothing).
-void dadt_nodes_shared(const double* nodes_mm, int n_nodes, const float* dip_packed, int n_dip,
-                       const double* transform_dev, int n_sets, double didt, float* out, cudaStream_t s,
-                       DevArray<float>& scratch);
 // The two direct sums on raw node coordinates with an explicit FP32 scale (1: the bare dipole sum).
 void dadt_zcoil_raw(const double* nodes_mm, int n_nodes, const void* zpacked, int n_dip, const double* transforms_dev,
                     int k, float scale, float* out, cudaStream_t s, int max_blocks = 0);
@@ -475,7 +467,12 @@ void adm_adjoint_rhs(const Mesh& m, const double* alpha, const AdmDirections& di
 void adm_node_weights(const Mesh& m, const double* lam, int K, const double* alpha, const AdmDirections& dirs,
                       double* W, cudaStream_t s);
 void adm_centred_nodes(const Mesh& m, const double* center_mm, double* out_m, cudaStream_t s);
-void adm_grid_points(const AdmGrid& gr, double* out /* (n_grid, 3) mm */, cudaStream_t s);
+// The reciprocity field Q (n_dir, n_grid, 3) of the nodal weights W (n_dir, n_nodes, 3) on a grid, every
+// direction in one pass over the sources (qfield.cu). sources holds them by axis, scratch the source runs' partial fields when
+// the grid alone does not fill the GPU (grown on demand and kept by the caller, so repeated calls
+// allocate nothing).
+void qfield_sample(const Mesh& m, const AdmGrid& gr, const double* W, int n_dir, float* Q, DevArray<double>& sources,
+                   DevArray<float>& scratch, int sm_count, cudaStream_t s);
 // E (P, n_dir) from the sampled field Q (n_dir, n_grid, 3); bad[3] receives, per axis, the smallest
 // flat sample index p * n_dip + j of a dipole off the grid (left untouched when none is).
 void adm_evaluate(const float* Q, int n_dir, const AdmGrid& gr, const double* pos, const double* mom, int n_dip,

@@ -1,0 +1,284 @@
+// The reciprocity field on a grid (reference adm/reciprocity.py:173-213):
+//     Q_d(g) = mu0/4pi sum_n W_dn x (g - r_n) / |g - r_n|^3,  mesh nodes r_n, up to three directions d.
+//
+// With w_gn = 1/|g - r_n|^3 and c the centre of a tile of grid points, W x (g - r) splits into
+// W x (g - c) - W x (r - c), so
+//     Q_d(g) = (sum_n w_gn W_dn) x (g - c) - sum_n w_gn (W_dn x (r_n - c)):
+// per pair of a grid point and a node the distance and six multiply-adds a direction, 8 + 6 n_dir FP32 operations and one
+// reciprocal square root, where the cross product of every pair takes 8 + 9 n_dir. The products W x (r - c) are formed
+// once per block and node.
+//
+// Precision: g - c, r - c and W x (r - c) are taken in FP64 before they are rounded to FP32, which leaves less error near
+// a node than coordinates centred on the whole grid; both sums carry the same w. A block's sums over kStage nodes are
+// added to running sums of their own, so that rounding does not grow with the number of nodes.
+//
+// Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 47.7 ms against 73.7 for a cross product a pair
+// (26 operations a pair at the pipe's rate: 39 ms); 332k by 52k with one direction: 8.5 ms against 10.6. The largest error
+// against 64 bits 8.5e-6 of the largest value, 1.9e-5 before. The matrix w on the tensor cores (tcgen05 kind::tf32, w in two
+// terms from tensor memory, the weights in three) took 48.9 and 13.8 ms: a block there forms w, hands it over and waits in
+// step, and the pairs' distances alone, no matrix instruction issued, took 45.
+#include <algorithm>
+#include <cmath>
+
+#include "internal.hpp"
+
+namespace cunibs {
+namespace {
+
+constexpr int kThreads = 128;
+constexpr int kPerThread = 4;                     // grid points a thread, as two pairs for the packed instructions
+constexpr int kPoints = kThreads * kPerThread;    // points of a block's tile
+constexpr int kStage = 128;                       // nodes staged at once
+constexpr int kResident = 4;                      // blocks an SM
+
+// A staged node: -(r - c) and one unused word, then W and W x (r - c) of each direction.
+template <int ND>
+constexpr int record_words() {
+    return (4 + 6 * ND + 3) / 4 * 4;
+}
+template <int ND>
+constexpr int smem_bytes() {
+    return static_cast<int>(sizeof(float)) * (kStage * record_words<ND>() + kPoints * 6 * ND);
+}
+
+__device__ __forceinline__ float rsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Boxes of t[0] x t[1] x t[2] <= kPoints grid points; n[a] of them along axis a.
+struct QTiles {
+    int t[3];
+    int n[3];
+};
+
+// Sources as the kernel reads them, one array per axis: positions in metres (3, n), then the weights of each
+// direction (n_dir, 3, n).
+__global__ void sources_kernel(const double* __restrict__ nodes_mm, const double* __restrict__ W, int n, int n_dir,
+                               double* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    for (int a = 0; a < 3; ++a) out[static_cast<long>(a) * n + i] = nodes_mm[3 * static_cast<long>(i) + a] * 1e-3;
+    for (int d = 0; d < n_dir; ++d)
+        for (int a = 0; a < 3; ++a)
+            out[(3L + 3 * d + a) * n + i] = W[3 * (static_cast<long>(d) * n + i) + a];
+}
+
+// Work item = (tile of grid points, run of sources): item = run * n_tiles + tile. With one run the scaled
+// field goes to out; with several the run's unscaled partial goes to part[run], and partial_sum_kernel
+// adds the runs in order. The runs depend on the sizes only, never on ND, and a direction's sums are the same
+// operations whatever ND.
+template <int ND>
+__global__ void __launch_bounds__(kThreads, kResident)
+    qfield_kernel(AdmGrid gr, QTiles tiles, int n_tiles, const double* __restrict__ src, int n_src, int run, float scale,
+                  float* __restrict__ out, float* __restrict__ part) {
+    constexpr int kWords = record_words<ND>(), kPairs = 3 * ND;
+    extern __shared__ __align__(16) float rec[];
+    float2* total = reinterpret_cast<float2*>(rec + kStage * kWords);  // [point][pair of sums][thread]
+    const int tile = blockIdx.x % n_tiles, r0 = blockIdx.x / n_tiles;
+    const int at[3] = {tile / (tiles.n[1] * tiles.n[2]) * tiles.t[0], tile / tiles.n[2] % tiles.n[1] * tiles.t[1],
+                       tile % tiles.n[2] * tiles.t[2]};
+    double center[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int extent = min(tiles.t[a], gr.shape[a] - at[a]);
+        center[a] = (gr.origin_mm[a] + gr.spacing_mm[a] * (at[a] + 0.5 * (extent - 1))) * 1e-3;
+    }
+    // Point p of the tile: its place relative to the centre, and its index in the grid (-1 past the tile).
+    auto point = [&](int p, float (&g)[3]) {
+        const int in[3] = {p / (tiles.t[1] * tiles.t[2]), p / tiles.t[2] % tiles.t[1], p % tiles.t[2]};
+        bool inside = p < tiles.t[0] * tiles.t[1] * tiles.t[2];
+        long index = 0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const int extent = min(tiles.t[a], gr.shape[a] - at[a]);
+            inside = inside && in[a] < extent;
+            const int i = at[a] + min(in[a], extent - 1);
+            g[a] = static_cast<float>((gr.origin_mm[a] + gr.spacing_mm[a] * i) * 1e-3 - center[a]);
+            index = index * gr.shape[a] + i;
+        }
+        return inside ? index : -1L;
+    };
+    float2 gx[2], gy[2], gz[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        float g0[3], g1[3];
+        point(threadIdx.x + 2 * q * kThreads, g0);
+        point(threadIdx.x + (2 * q + 1) * kThreads, g1);
+        gx[q] = make_float2(g0[0], g1[0]);
+        gy[q] = make_float2(g0[1], g1[1]);
+        gz[q] = make_float2(g0[2], g1[2]);
+    }
+    for (int c = 0; c < kPerThread * kPairs; ++c) total[c * kThreads + threadIdx.x] = make_float2(0.f, 0.f);
+    const int j_begin = r0 * run, j_end = min(n_src, j_begin + run);
+    for (int j0 = j_begin; j0 < j_end; j0 += kStage) {
+        const int nt = min(kStage, j_end - j0);
+        __syncthreads();
+        for (int j = threadIdx.x; j < nt; j += kThreads) {
+            float* r = rec + j * kWords;
+            double x[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                x[a] = src[static_cast<long>(a) * n_src + j0 + j] - center[a];
+                r[a] = -static_cast<float>(x[a]);
+            }
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                double m[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) m[a] = src[(3L + 3 * d + a) * n_src + j0 + j];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const int u = (a + 1) % 3, v = (a + 2) % 3;
+                    r[4 + 6 * d + a] = static_cast<float>(m[a]);
+                    r[7 + 6 * d + a] = static_cast<float>(m[u] * x[v] - m[v] * x[u]);
+                }
+            }
+        }
+        __syncthreads();
+        float2 acc[kPerThread][kPairs];
+#pragma unroll
+        for (int u = 0; u < kPerThread; ++u)
+#pragma unroll
+            for (int c = 0; c < kPairs; ++c) acc[u][c] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int j = 0; j < nt; ++j) {
+            const float* r = rec + j * kWords;
+            const float4 at4 = *reinterpret_cast<const float4*>(r);
+            float wu[kPerThread];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float2 dx = __fadd2_rn(gx[q], make_float2(at4.x, at4.x));
+                const float2 dy = __fadd2_rn(gy[q], make_float2(at4.y, at4.y));
+                const float2 dz = __fadd2_rn(gz[q], make_float2(at4.z, at4.z));
+                float2 d2 = __fmul2_rn(dx, dx);
+                d2 = __ffma2_rn(dy, dy, d2);
+                d2 = __ffma2_rn(dz, dz, d2);
+                const float2 inv = make_float2(rsqrt_fast(d2.x), rsqrt_fast(d2.y));
+                const float2 w = __fmul2_rn(__fmul2_rn(inv, inv), inv);
+                wu[2 * q] = w.x;
+                wu[2 * q + 1] = w.y;
+            }
+#pragma unroll
+            for (int c = 0; c < kPairs; ++c) {
+                const float2 m = *reinterpret_cast<const float2*>(r + 4 + 2 * c);
+#pragma unroll
+                for (int u = 0; u < kPerThread; ++u) acc[u][c] = __ffma2_rn(make_float2(wu[u], wu[u]), m, acc[u][c]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kPerThread; ++u)
+#pragma unroll
+            for (int c = 0; c < kPairs; ++c) {
+                float2* t = total + (u * kPairs + c) * kThreads + threadIdx.x;
+                *t = __fadd2_rn(*t, acc[u][c]);
+            }
+    }
+    const long count = static_cast<long>(gr.shape[0]) * gr.shape[1] * gr.shape[2];
+    float* o = part ? part + static_cast<long>(r0) * ND * count * 3 : out;
+    const float sc = part ? 1.0f : scale;
+#pragma unroll 1
+    for (int u = 0; u < kPerThread; ++u) {
+        float g[3];
+        const long index = point(threadIdx.x + u * kThreads, g);
+        if (index < 0) continue;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            const float2* t = total + (u * kPairs + 3 * d) * kThreads + threadIdx.x;
+            const float2 t0 = t[0], t1 = t[kThreads], t2 = t[2 * kThreads];
+            const float m[3] = {t0.x, t0.y, t1.x}, w[3] = {t1.y, t2.x, t2.y};
+            float* q = o + (static_cast<long>(d) * count + index) * 3;
+            q[0] = sc * (fmaf(m[1], g[2], -m[2] * g[1]) - w[0]);
+            q[1] = sc * (fmaf(m[2], g[0], -m[0] * g[2]) - w[1]);
+            q[2] = sc * (fmaf(m[0], g[1], -m[1] * g[0]) - w[2]);
+        }
+    }
+}
+
+// out = scale * (the runs' partials added in order).
+__global__ void partial_sum_kernel(long count, int runs, const float* __restrict__ part, float scale,
+                                   float* __restrict__ out) {
+    const long q = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q >= count) return;
+    float v = part[q];
+    for (int c = 1; c < runs; ++c) v += part[c * count + q];
+    out[q] = scale * v;
+}
+
+// The box of at most kPoints points that covers the grid with the fewest tiles, compact first on ties
+// (the lever arm |g - c| multiplies the sums' rounding): sides up to 32, the longest at most four times the
+// shortest side that is not the whole axis.
+QTiles choose_tiles(const AdmGrid& gr) {
+    QTiles best{};
+    double best_cost = INFINITY;
+    for (int x = 1; x <= 32; ++x)
+        for (int y = 1; y <= 32; ++y) {
+            if (x * y > kPoints) break;
+            const int z = std::min(32, kPoints / (x * y));
+            const int t[3] = {std::min(x, gr.shape[0]), std::min(y, gr.shape[1]), std::min(z, gr.shape[2])};
+            double n = 1.0, lever = 0.0;
+            for (int a = 0; a < 3; ++a) {
+                n *= (gr.shape[a] + t[a] - 1) / t[a];
+                lever += (t[a] * gr.spacing_mm[a]) * (t[a] * gr.spacing_mm[a]);
+            }
+            const double cube = 3.0 * std::pow(kPoints * gr.spacing_mm[0] * gr.spacing_mm[1] * gr.spacing_mm[2], 2.0 / 3.0);
+            if (lever > 2.25 * cube && x * y * z > 1 && best_cost < INFINITY) continue;  // at most 1.5 times a cube's diagonal
+            const double cost = n * (1.0 + 0.02 * lever / cube);
+            if (cost < best_cost) {
+                best_cost = cost;
+                for (int a = 0; a < 3; ++a) best.t[a] = t[a];
+            }
+        }
+    for (int a = 0; a < 3; ++a) best.n[a] = (gr.shape[a] + best.t[a] - 1) / best.t[a];
+    return best;
+}
+
+}  // namespace
+
+void qfield_sample(const Mesh& m, const AdmGrid& gr, const double* W, int n_dir, float* Q, DevArray<double>& sources,
+                   DevArray<float>& scratch, int sm_count, cudaStream_t s) {
+    if (n_dir < 1 || n_dir > kAdmMaxDir) fail(kEInval, "between 1 and 3 adjoint directions");
+    sources.reserve(3 * static_cast<std::size_t>(m.n_nodes) * (1 + n_dir));
+    sources_kernel<<<grid_for(m.n_nodes), kBlock, 0, s>>>(m.nodes.get(), W, m.n_nodes, n_dir, sources.get());
+    count_launch();
+    const QTiles tiles = choose_tiles(gr);
+    const int n_tiles = tiles.n[0] * tiles.n[1] * tiles.n[2];
+    // Runs of sources so that the last wave of blocks (kResident per SM) is nearly full: the fewest that reach
+    // 97% of whole waves, else the best of 16; a run holds at least 1024 sources.
+    const int slots = sm_count * kResident;
+    int runs = 1;
+    double best = 0.0;
+    for (int c = 1; c <= std::max(1, std::min(16, m.n_nodes / 1024)); ++c) {
+        const double items = static_cast<double>(n_tiles) * c;
+        const double full = items / (std::ceil(items / slots) * slots);
+        if (full > best + 1e-9) {
+            best = full;
+            runs = c;
+        }
+        if (full >= 0.97) break;
+    }
+    const int run = ((m.n_nodes + runs - 1) / runs + kStage - 1) / kStage * kStage;
+    runs = (m.n_nodes + run - 1) / run;
+    const long count = static_cast<long>(gr.shape[0]) * gr.shape[1] * gr.shape[2] * 3 * n_dir;
+    if (runs > 1) scratch.reserve(static_cast<std::size_t>(count) * runs);
+    float* part = runs > 1 ? scratch.get() : nullptr;
+    auto go = [&](auto nd) {
+        constexpr int ND = decltype(nd)::value;
+        CUNIBS_CHECK(cudaFuncSetAttribute(qfield_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<ND>()));
+        qfield_kernel<ND><<<n_tiles * runs, kThreads, smem_bytes<ND>(), s>>>(gr, tiles, n_tiles, sources.get(), m.n_nodes,
+                                                                             run, 1e-7f, Q, part);
+        count_launch();
+    };
+    if (n_dir == 1) go(std::integral_constant<int, 1>{});
+    else if (n_dir == 2) go(std::integral_constant<int, 2>{});
+    else go(std::integral_constant<int, 3>{});
+    CUNIBS_LAUNCH_CHECK("reciprocity field");
+    if (runs > 1) {
+        partial_sum_kernel<<<grid_for(count), kBlock, 0, s>>>(count, runs, part, 1e-7f, Q);
+        count_launch();
+    }
+    CUNIBS_LAUNCH_CHECK("reciprocity field sum");
+}
+
+}  // namespace cunibs
