@@ -614,7 +614,7 @@ __global__ void compose_kernel(int* __restrict__ agg, const int* __restrict__ st
 // GPU idle between two steps.
 // Measured on the 6,763 rows of a 0.68M-tet head's level 1: with the pivot block inverted by a launch of its
 // own (0.21 ms of one block) and 64 x 64 update tiles of 4 x 4 patches staged in two halves (0.25 ms a step),
-// 56 ms; set-up to the first result 89-95 ms, 54 ms with this form.
+// 56 ms; set-up to the first result 89-95 ms, 54 ms with the chain inside the update and 128 x 64 tiles.
 
 constexpr int kSweepB = 64;
 constexpr int kSweepRows = 128;  // rows of an update tile (two blocks), by kSweepB columns
@@ -764,12 +764,28 @@ __device__ __forceinline__ void sweep_copy16(double* smem, const double* gmem) {
                  : "memory");
 }
 
+// d += a b for 16 x 8 x 16 FP64 operands spread over the warp (g = lane / 4, t = lane % 4): a[i] = A[g + 8 (i % 2)]
+// [t + 4 (i / 2)], b[i] = B[t + 4 i][g], d[0..1] = D[g][2 t ..], d[2..3] = D[g + 8][2 t ..].
+__device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[8], const double (&b)[4]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, "
+        "{%0,%1,%2,%3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]),
+          "d"(b[2]), "d"(b[3]));
+}
+
 // A_IJ -= C_I A_kJ for the tiles (128 rows x 64 columns, row block I of two blocks) that meet the lower block
-// triangle, blocks k left alone. Bound by the FP64 pipe (n^2 kSweepB / 2 multiply-adds a step) with the tile's
-// read and write beside it: both operands sit k-major in shared memory (96 KB, two blocks an SM, so one
-// block's copies run under the other's arithmetic), and a thread's 8 x 4 patch takes 6 16-byte
-// shared-memory loads per 32 multiply-adds. Tile t of the list: I(I + 1) <= t, J = t - I(I + 1).
-constexpr std::size_t kUpdateSmem = sizeof(double) * kSweepB * (kSweepRows + kSweepB);
+// triangle, blocks k left alone. Bound by the FP64 units (n^2 kSweepB / 2 multiply-adds a step) with the tile's
+// read and write beside them. The products run on the FP64 matrix instruction (tcgen05 has no FP64 kind), whose rate is
+// that of the scalar pipe: what it saves is shared memory, where a scalar 8 x 4 patch a thread reads 6 16-byte pieces per
+// 32 multiply-adds and the warp's 32 x 32 patch an eighth of that. Both operands sit k-major in rows of 8 doubles over a
+// multiple of 16, which spreads a fragment over all banks (104 KB, two blocks an SM, so one block's copies run under the
+// other's arithmetic); rows of 4 over measure the same. On 6,763 rows a step takes 0.127 ms, 0.171 with scalar patches
+// (its arithmetic at the pipe's rate: 0.08; set-up to the first result 48.2 -> 41.4 ms).
+// Tile t of the list: I(I + 1) <= t, J = t - I(I + 1).
+constexpr int kUpdateLdx = kSweepRows + 8, kUpdateLdy = kSweepB + 8;
+constexpr std::size_t kUpdateSmem = sizeof(double) * kSweepB * (kUpdateLdx + kUpdateLdy);
 
 __global__ void __launch_bounds__(256, 2) sweep_update_kernel(double* __restrict__ m, int N, int k,
                                                              const double* __restrict__ cbuf,
@@ -777,7 +793,7 @@ __global__ void __launch_bounds__(256, 2) sweep_update_kernel(double* __restrict
                                                              double* __restrict__ pinv_next, int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char sweep_smem[];
     double* xs = reinterpret_cast<double*>(sweep_smem);  // C_I^T, 64 x 128
-    double* ys = xs + kSweepB * kSweepRows;              // A_kJ, 64 x 64
+    double* ys = xs + kSweepB * kUpdateLdx;              // A_kJ, 64 x 64
     const int T = N / kSweepB;
     // The tile that holds the next pivot block goes first.
     const int next = k + 1;
@@ -793,62 +809,77 @@ __global__ void __launch_bounds__(256, 2) sweep_update_kernel(double* __restrict
     for (int q = threadIdx.x; q < kSweepB * (kSweepRows / 2); q += blockDim.x) {
         const int r = q / (kSweepRows / 2), c = q % (kSweepRows / 2) * 2;
         if (c < kSweepB || half1)
-            sweep_copy16(xs + r * kSweepRows + c, cbuf + static_cast<long>(r) * N + static_cast<long>(I) * kSweepRows + c);
+            sweep_copy16(xs + r * kUpdateLdx + c, cbuf + static_cast<long>(r) * N + static_cast<long>(I) * kSweepRows + c);
     }
     for (int q = threadIdx.x; q < kSweepB * (kSweepB / 2); q += blockDim.x) {
         const int r = q / (kSweepB / 2), c = q % (kSweepB / 2) * 2;
-        sweep_copy16(ys + r * kSweepB + c, rbuf + static_cast<long>(r) * N + static_cast<long>(J) * kSweepB + c);
+        sweep_copy16(ys + r * kUpdateLdy + c, rbuf + static_cast<long>(r) * N + static_cast<long>(J) * kSweepB + c);
+    }
+    // The tile itself, towards L2 meanwhile: a row of it is four 128-byte lines.
+    for (int q = threadIdx.x; q < kSweepRows * 4; q += blockDim.x) {
+        const int bi = 2 * I + q / (kSweepB * 4);
+        if (bi < T && bi != k && bi >= J)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(m + (static_cast<long>(I) * kSweepRows + q / 4) * N +
+                                                         static_cast<long>(J) * kSweepB + q % 4 * 16));
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // A thread's rows: 4 ty .. 4 ty + 3 of both 64-row halves.
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+    // A warp's patch: 32 rows of one 64-row half by 32 columns, in 2 x 4 fragments of 16 x 8.
+    const int warp = threadIdx.x / 32, g = threadIdx.x % 32 / 4, lane4 = threadIdx.x % 4;
+    const int wr = warp / 2 * 32, wc = warp % 2 * 32;
+    const int bi = 2 * I + warp / 4;
+    const bool mine = bi < T && bi != k && bi >= J;  // bi < J: above the block diagonal
     double acc[2][4][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int b = 0; b < 4; ++b)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[h][a][b] = 0.0;
-#pragma unroll 4
-    for (int kk = 0; kk < kSweepB; ++kk) {
-        const double2 y0 = *reinterpret_cast<const double2*>(ys + kk * kSweepB + tx * 4);
-        const double2 y1 = *reinterpret_cast<const double2*>(ys + kk * kSweepB + tx * 4 + 2);
-        const double yb[4] = {y0.x, y0.y, y1.x, y1.y};
+            for (int i = 0; i < 4; ++i) acc[a][b][i] = 0.0;
+    if (mine) {
+#pragma unroll 1
+        for (int kk = 0; kk < kSweepB; kk += 16) {
+            const double* x = xs + (kk + lane4) * kUpdateLdx + wr + g;
+            const double* y = ys + (kk + lane4) * kUpdateLdy + wc + g;
+            double fa[2][8];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const double* x = xs + kk * kSweepRows + h * kSweepB + ty * 4;
-            const double2 x0 = *reinterpret_cast<const double2*>(x), x1 = *reinterpret_cast<const double2*>(x + 2);
-            const double xa[4] = {x0.x, x0.y, x1.x, x1.y};
+            for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+                for (int i = 0; i < 8; ++i) fa[a][i] = x[i / 2 * 4 * kUpdateLdx + a * 16 + i % 2 * 8];
 #pragma unroll
-                for (int b = 0; b < 4; ++b) acc[h][a][b] = fma(xa[a], yb[b], acc[h][a][b]);
+            for (int b = 0; b < 4; ++b) {
+                double fb[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) fb[i] = y[i * 4 * kUpdateLdy + b * 8];
+                mma_f64(acc[0][b], fa[0], fb);
+                mma_f64(acc[1][b], fa[1], fb);
+            }
         }
     }
     if (pivot) __syncthreads();  // xs is about to hold the pivot block
+    if (mine) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int bi = 2 * I + h;
-        if (bi >= T || bi == k || bi < J) continue;  // bi < J: above the block diagonal
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            double* row = m + (static_cast<long>(bi) * kSweepB + ty * 4 + a) * N + static_cast<long>(J) * kSweepB + tx * 4;
-            double2 v0 = *reinterpret_cast<double2*>(row), v1 = *reinterpret_cast<double2*>(row + 2);
-            v0.x -= acc[h][a][0];
-            v0.y -= acc[h][a][1];
-            v1.x -= acc[h][a][2];
-            v1.y -= acc[h][a][3];
-            *reinterpret_cast<double2*>(row) = v0;
-            *reinterpret_cast<double2*>(row + 2) = v1;
-            if (pivot && bi == next) {
-                double* p = xs + (ty * 4 + a) * (kSweepB + 1) + tx * 4;
-                p[0] = v0.x;
-                p[1] = v0.y;
-                p[2] = v1.x;
-                p[3] = v1.y;
+            for (int h = 0; h < 2; ++h) {
+                const int r = wr + a * 16 + h * 8 + g;
+                double* row = m + (static_cast<long>(I) * kSweepRows + r) * N + static_cast<long>(J) * kSweepB;
+                double2 v[4];
+#pragma unroll
+                for (int b = 0; b < 4; ++b) v[b] = *reinterpret_cast<double2*>(row + wc + b * 8 + 2 * lane4);
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const int c = wc + b * 8 + 2 * lane4;
+                    v[b].x -= acc[a][b][2 * h];
+                    v[b].y -= acc[a][b][2 * h + 1];
+                    *reinterpret_cast<double2*>(row + c) = v[b];
+                    if (pivot && bi == next) {
+                        double* p = xs + (r % kSweepB) * (kSweepB + 1) + c;
+                        p[0] = v[b].x;
+                        p[1] = v[b].y;
+                    }
+                }
             }
-        }
     }
     if (pivot) {
         __syncthreads();
