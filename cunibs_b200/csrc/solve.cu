@@ -1288,11 +1288,17 @@ class Solver {
     const Hierarchy* h = nullptr;
     int n = 0;
     int kcap = 0;
-    // Solve-loop kernels launched with programmatic stream serialization (pdl_enter): off by default,
-    // on with CUNIBS_PROGRAMMATIC_LAUNCH=1. With the V-cycle's bottom at level 1 the loop is mostly
-    // multi-wave finest-level kernels, whose early-resident successors take their later waves'
-    // slots: split solve 3.38 ms per block of 8 with it, 3.26 ms without.
-    bool pdl = false;
+    // Whether the solve loop's kernels are launched with programmatic stream serialization (pdl_enter), so that a
+    // kernel's launch overlaps its predecessor. That pays where the loop is a chain of launches: the finest level's rows and
+    // columns at no more than 256 threads an SM (one placement on 16k rows 909 -> 880 us). Above, the successors'
+    // waiting blocks take slots and issue from kernels that fill the SMs: one placement on 121k rows 1457 -> 1494 us,
+    // optimisation on 52k rows 10.73 -> 10.80 ms, blocks of 8 on 52k rows 4.20 -> 4.26 ms and on 179k rows (split solve)
+    // 3.26 -> 3.38 ms. CUNIBS_PROGRAMMATIC_LAUNCH=0 or 1 decides for every size.
+    int launch_mode = -1;
+    template <int K>
+    bool dependent() const {
+        return launch_mode >= 0 ? launch_mode == 1 : static_cast<long>(n) * K <= static_cast<long>(sm_count) * 256;
+    }
     // Columns per lane of the one-lane-per-row operators (the *_cols kernels; bitwise the same
     // results): 2 by default, CUNIBS_LANE_COLUMNS=1 or 4 to choose.
     int lane_cols = 2;
@@ -1588,7 +1594,7 @@ void Solver::dense_bottom(const T* b, T* x) {
     cfg.numAttrs = 0;
     CUNIBS_CHECK(cudaLaunchKernelEx(&cfg, dense_part_kernel<T, K>, nb, dense_ld(nb), g.cols, g.split_rows, cinv<T>(), b,
                                     part));
-    launch_loop(pdl, dense_sum_kernel<T, K>, grid_for(static_cast<std::int64_t>(nb) * K), kBlock, stream, nb, g.splits,
+    launch_loop(dependent<K>(), dense_sum_kernel<T, K>, grid_for(static_cast<std::int64_t>(nb) * K), kBlock, stream, nb, g.splits,
                 static_cast<const T*>(part), x);
     count_launch(2);
 }
@@ -1618,11 +1624,11 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
         if (lv.tpr_a == 1 && dispatch_cols<K>(cols, [&](auto cc_) {
                 constexpr int C = decltype(cc_)::value;
                 if constexpr (std::is_same<T, double>::value && C == 4) {
-                    launch_loop(pdl, cheby_cols_kernel<T, K, 2>, col_grid<K, 2>(lv.n), kColBlock, s, lv.n,
+                    launch_loop(dependent<K>(), cheby_cols_kernel<T, K, 2>, col_grid<K, 2>(lv.n), kColBlock, s, lv.n,
                                 lv.a.ptr.get(), lv.a.col.get(), lval<T>(l), ldinv<T>(l), bi, cur, prev, cc, cp, al,
                                 out);
                 } else {
-                    launch_loop(pdl, cheby_cols_kernel<T, K, C>, col_grid<K, C>(lv.n), kColBlock, s, lv.n,
+                    launch_loop(dependent<K>(), cheby_cols_kernel<T, K, C>, col_grid<K, C>(lv.n), kColBlock, s, lv.n,
                                 lv.a.ptr.get(), lv.a.col.get(), lval<T>(l), ldinv<T>(l), bi, cur, prev, cc, cp, al,
                                 out);
                 }
@@ -1633,7 +1639,7 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
         if (lv.tpr_a > 1 && dispatch_subcols<K>(lv.tpr_a, cols, [&](auto tc, auto cc_) {
                 constexpr int TPR = decltype(tc)::value;
                 constexpr int C = decltype(cc_)::value;
-                launch_loop(pdl, cheby_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n), kColBlock, s, lv.n,
+                launch_loop(dependent<K>(), cheby_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n), kColBlock, s, lv.n,
                             lv.a.ptr.get(), lv.a.col.get(), lval<T>(l), ldinv<T>(l), bi, cur, prev, cc, cp, al, out);
             })) {
             count_launch();
@@ -1641,7 +1647,7 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
         }
         dispatch_tpr<K>(lv.tpr_a, [&](auto tc) {
             constexpr int TPR = decltype(tc)::value;
-            launch_loop(pdl, cheby_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n), Group<K, TPR>::kBlock, s, lv.n,
+            launch_loop(dependent<K>(), cheby_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n), Group<K, TPR>::kBlock, s, lv.n,
                         lv.a.ptr.get(), lv.a.col.get(), lval<T>(l), ldinv<T>(l), bi, cur, prev, cc, cp, al, out);
         });
         count_launch();
@@ -1669,7 +1675,7 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
                 const Level& lv = H.levels[0];
                 dispatch_tpr<K>(lv.tpr_a, [&](auto tc) {
                     constexpr int TPR = decltype(tc)::value;
-                    launch_loop(pdl, cheby_dot_kernel<T, K, TPR>, reduce_grid_rows<TPR>(lv.n),
+                    launch_loop(dependent<K>(), cheby_dot_kernel<T, K, TPR>, reduce_grid_rows<TPR>(lv.n),
                                 TPR == 1 ? reduce_threads<K>(lv.n) : TT, s, lv.n,
                                 lv.a.ptr.get(), lv.a.col.get(), lval<T>(0), ldinv<T>(0), bi, cur, prev,
                                 static_cast<T>(ch.c_cur[st - 1]), cp, static_cast<T>(ch.alpha[st - 1]), out,
@@ -1694,7 +1700,7 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
         T* other = odd ? w.r[l].get() : w.x[l].get();
         const unsigned g = n_tiles(lv.n);
         if (l == 0 && !jz_done) {
-            launch_loop(pdl, jz_kernel<T, K>, g, TT, s, lv.n, ldinv<T>(0), bi, static_cast<T>(ch.alpha0), first);
+            launch_loop(dependent<K>(), jz_kernel<T, K>, g, TT, s, lv.n, ldinv<T>(0), bi, static_cast<T>(ch.alpha0), first);
             count_launch();
         }
         sweep(l, bi, nullptr, first, other, nullptr);
@@ -1702,19 +1708,19 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
             (lv.tpr_a == 1 && dispatch_cols<K>(cols, [&](auto cc_) {
                  constexpr int C =
                      (std::is_same<T, double>::value && decltype(cc_)::value == 4) ? 2 : decltype(cc_)::value;
-                 launch_loop(pdl, residual_cols_kernel<T, K, C>, col_grid<K, C>(lv.n), kColBlock, s, lv.n,
+                 launch_loop(dependent<K>(), residual_cols_kernel<T, K, C>, col_grid<K, C>(lv.n), kColBlock, s, lv.n,
                              lv.a.ptr.get(), lv.a.col.get(), lval<T>(l), w.x[l].get(), bi, w.r[l].get());
              })) ||
             (lv.tpr_a > 1 && dispatch_subcols<K>(lv.tpr_a, cols, [&](auto tc, auto cc_) {
                  constexpr int TPR = decltype(tc)::value;
                  constexpr int C = decltype(cc_)::value;
-                 launch_loop(pdl, residual_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n), kColBlock, s,
+                 launch_loop(dependent<K>(), residual_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n), kColBlock, s,
                              lv.n, lv.a.ptr.get(), lv.a.col.get(), lval<T>(l), w.x[l].get(), bi, w.r[l].get());
              }));
         if (!grouped) {
             dispatch_tpr<K>(lv.tpr_a, [&](auto tc) {
                 constexpr int TPR = decltype(tc)::value;
-                launch_loop(pdl, residual_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n), Group<K, TPR>::kBlock, s,
+                launch_loop(dependent<K>(), residual_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n), Group<K, TPR>::kBlock, s,
                             lv.n, lv.a.ptr.get(), lv.a.col.get(), lval<T>(l), w.x[l].get(), bi, w.r[l].get());
             });
         }
@@ -1731,13 +1737,13 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
         const bool rgrouped = lv.tpr_r > 1 && dispatch_subcols<K>(lv.tpr_r, cols, [&](auto tc, auto cc_) {
             constexpr int TPR = decltype(tc)::value;
             constexpr int C = decltype(cc_)::value;
-            launch_loop(pdl, restrict_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n_coarse), kColBlock, s,
+            launch_loop(dependent<K>(), restrict_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n_coarse), kColBlock, s,
                         lv.n_coarse, lv.r.ptr.get(), lv.r.col.get(), rval<T>(l), w.r[l].get(), nb, nd,
                         static_cast<T>(ch.alpha0), nx);
         });
         if (!rgrouped) dispatch_tpr<K>(lv.tpr_r, [&](auto tc) {
             constexpr int TPR = decltype(tc)::value;
-            launch_loop(pdl, restrict_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n_coarse), Group<K, TPR>::kBlock, s,
+            launch_loop(dependent<K>(), restrict_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n_coarse), Group<K, TPR>::kBlock, s,
                         lv.n_coarse, lv.r.ptr.get(), lv.r.col.get(), rval<T>(l), w.r[l].get(), nb, nd,
                         static_cast<T>(ch.alpha0), nx);
         });
@@ -1753,19 +1759,19 @@ bool Solver::vcycle(const T* b, T* z, bool jz_done, bool dot) {
             (lv.tpr_p == 1 && dispatch_cols<K>(cols, [&](auto cc_) {
                  constexpr int C =
                      (std::is_same<T, double>::value && decltype(cc_)::value == 4) ? 2 : decltype(cc_)::value;
-                 launch_loop(pdl, prolong_cols_kernel<T, K, C>, col_grid<K, C>(lv.n), kColBlock, s, lv.n,
+                 launch_loop(dependent<K>(), prolong_cols_kernel<T, K, C>, col_grid<K, C>(lv.n), kColBlock, s, lv.n,
                              lv.p.ptr.get(), lv.p.col.get(), pval<T>(l), xc, w.x[l].get());
              })) ||
             (lv.tpr_p > 1 && dispatch_subcols<K>(lv.tpr_p, cols, [&](auto tc, auto cc_) {
                  constexpr int TPR = decltype(tc)::value;
                  constexpr int C = decltype(cc_)::value;
-                 launch_loop(pdl, prolong_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n), kColBlock, s,
+                 launch_loop(dependent<K>(), prolong_subcols_kernel<T, K, TPR, C>, subcol_grid<K, TPR, C>(lv.n), kColBlock, s,
                              lv.n, lv.p.ptr.get(), lv.p.col.get(), pval<T>(l), xc, w.x[l].get());
              }));
         if (!grouped) {
             dispatch_tpr<K>(lv.tpr_p, [&](auto tc) {
                 constexpr int TPR = decltype(tc)::value;
-                launch_loop(pdl, prolong_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n), Group<K, TPR>::kBlock, s,
+                launch_loop(dependent<K>(), prolong_kernel<T, K, TPR>, group_grid<K, TPR>(lv.n), Group<K, TPR>::kBlock, s,
                             lv.n, lv.p.ptr.get(), lv.p.col.get(), pval<T>(l), xc, w.x[l].get());
             });
         }
@@ -1839,7 +1845,7 @@ void Solver::pcg_tail(TZ* r_v, TZ* z, bool jz_done) {
     constexpr int TT = tile_threads<K>();
     const bool fused = vcycle<TZ, K>(r_v, z, jz_done, true);
     if (!fused) {
-        launch_loop(pdl, dot_beta_kernel<TZ, K>, reduce_grid(n), TT, stream, n, r_v, z, partials.get(), counter.get(),
+        launch_loop(dependent<K>(), dot_beta_kernel<TZ, K>, reduce_grid(n), TT, stream, n, r_v, z, partials.get(), counter.get(),
                     rz.get(), frozen.get(), beta.get());
         count_launch();
     }
@@ -1853,14 +1859,14 @@ void Solver::pcg_iteration(const int* ptr, const int* col, const T* val, T* x, T
     const unsigned g = reduce_grid(n);
     dispatch_tpr<K>(tpr0(), [&](auto tc) {
         constexpr int TPR = decltype(tc)::value;
-        launch_loop(pdl, spmv_alpha_kernel<T, TZ, K, TPR>, reduce_grid_rows<TPR>(n),
+        launch_loop(dependent<K>(), spmv_alpha_kernel<T, TZ, K, TPR>, reduce_grid_rows<TPR>(n),
                     TPR == 1 ? reduce_threads<K>(n) : TT, stream, n, ptr, col, val, z,
                     p, ap, partials.get(), counter.get(), rz.get(), beta.get(), frozen.get(), alpha.get());
     });
     count_launch();
     const bool has_levels = !h->levels.empty();
     constexpr bool narrow = !std::is_same<T, TZ>::value;
-    launch_loop(pdl, update_xr_kernel<T, TZ, K>, g, reduce_threads<K>(n), stream, n, alpha.get(), p, ap, x, r, partials.get(),
+    launch_loop(dependent<K>(), update_xr_kernel<T, TZ, K>, g, reduce_threads<K>(n), stream, n, alpha.get(), p, ap, x, r, partials.get(),
                 counter.get(), ref, tol, tol_vec, frozen.get(), iter_counter.get(), conv_iter.get(), rel.get(), record,
                 has_levels ? ldinv<TZ>(0) : nullptr, static_cast<TZ>(h->cheby.alpha0),
                 has_levels ? first0<TZ>() : nullptr, narrow ? r_v : nullptr, loop, use_loop, cap.get());
@@ -2035,7 +2041,7 @@ SolverPtr make_solver(const Hierarchy& h, const Params& p) {
     const char* host_loop = std::getenv("CUNIBS_SOLVER_HOST_LOOP");
     sv->while_unsupported = host_loop != nullptr && host_loop[0] == '1';
     const char* pdl = std::getenv("CUNIBS_PROGRAMMATIC_LAUNCH");
-    sv->pdl = pdl != nullptr && pdl[0] == '1';
+    if (pdl != nullptr && (pdl[0] == '0' || pdl[0] == '1')) sv->launch_mode = pdl[0] - '0';
     const char* lanes = std::getenv("CUNIBS_LANE_COLUMNS");
     if (lanes != nullptr && (lanes[0] == '1' || lanes[0] == '2' || lanes[0] == '4')) sv->lane_cols = lanes[0] - '0';
     int dev = 0;

@@ -64,3 +64,28 @@ def test_groups_of_tiles_leave_the_sums_as_they_are(spacing, precision):
             np.testing.assert_array_equal(itk, it[:k])
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("spacing", [11.0, 5.2, 4.2])
+@pytest.mark.parametrize("precision", [_native.PREC_SPLIT, _native.PREC_PLAIN_FP64])
+def test_launch_modes_give_the_same_bits(spacing, precision, monkeypatch):
+    """Programmatic launches on, off and by the rule (on up to 256 rows and columns an SM: 2k rows at 16
+    columns, 21k at one; off at 21k and 45k at two)."""
+    m = sphere_head(spacing, 90.0, jitter_mm=0.2, seed=2)
+    got = {}
+    for mode in ("0", "1", None):
+        if mode is None:
+            monkeypatch.delenv("CUNIBS_PROGRAMMATIC_LAUNCH", raising=False)
+        else:
+            monkeypatch.setenv("CUNIBS_PROGRAMMATIC_LAUNCH", mode)
+        ctx = _native.Context(m.nodes_mm, m.tet_nodes, m.tet_tags, m.skin_tris, _native.default_params())
+        try:
+            b = np.random.default_rng(6).standard_normal((ctx.array("a_ptr", 0).shape[0] - 1, 16))
+            got[mode] = [ctx.solve(np.ascontiguousarray(b[:, :k]), k, k, precision=precision, tolerance=TOL)[:2]
+                         for k in (1, 2, 16)]
+        finally:
+            ctx.close()
+    for mode in ("1", None):
+        for (x, it), (x0, it0) in zip(got[mode], got["0"]):
+            np.testing.assert_array_equal(x, x0)
+            np.testing.assert_array_equal(it, it0)
