@@ -114,12 +114,14 @@ __device__ __forceinline__ void final_reduce(const double* __restrict__ partials
 // in order (predicated off past the row's end). One lane per row (S = 1, the finest levels) takes
 // the plain loop: measured on the 1M-tet operator (178k rows, ~15 entries per row, 8 columns) the
 // batches of 4, 8, 12 and 16 cost registers and occupancy for more than the chains they put in
-// flight (PCG iteration 0.266 ms at 8, 0.247 ms plain). Both keep the plain loop's order of
-// additions, so the result does not depend on the batch.
-template <typename T, int S, typename TX = T>
+// flight (PCG iteration 0.266 ms at 8, 0.247 ms plain). A block of one column (NARROW) has a thread a row and leaves
+// the GPU short of threads, so registers are free and it takes eight too: one placement on 16k rows 881 -> 845 us, on
+// 121k rows 1454 -> 1434, on 440k rows the same; 16 at a time 839, 1463 and 6% slower on 440k. All keep the plain
+// loop's order of additions, so the result does not depend on the batch.
+template <typename T, int S, typename TX = T, bool NARROW = false>
 __device__ __forceinline__ T strided_dot(const int* __restrict__ col, const T* __restrict__ val,
                                          const TX* __restrict__ x, int p, int e, long ld, int c, T acc) {
-    constexpr int B = S == 1 ? 1 : 8;
+    constexpr int B = S > 1 ? 8 : (NARROW ? 8 : 1);
     for (; p < e; p += B * S) {
         int cj[B];
         T vj[B];
@@ -198,7 +200,7 @@ __device__ __forceinline__ T group_row_dot(const int* __restrict__ ptr, const in
                                            const T* __restrict__ val, const TX* __restrict__ x, int row, int r,
                                            int sub, int c, bool valid) {
     T acc = T(0);
-    if (valid) acc = strided_dot<T, TPR, TX>(col, val, x, ptr[row] + sub, ptr[row + 1], K, c, acc);
+    if (valid) acc = strided_dot<T, TPR, TX, K == 1>(col, val, x, ptr[row] + sub, ptr[row + 1], K, c, acc);
     if constexpr (TPR == 1) {
         return acc;
     } else if constexpr (TPR * K <= kWarp) {
@@ -999,7 +1001,7 @@ __global__ void __launch_bounds__(TPR == 1 ? grouped_threads<K>() : tile_threads
     double v = 0.0;
     if constexpr (TPR == 1) {
         v = run_tiles<K>(n, [&](int row, int) {
-            return direction(row, strided_dot<T, 1, TZ>(col, val, z, ptr[row], ptr[row + 1], K, c, T(0)));
+            return direction(row, strided_dot<T, 1, TZ, K == 1>(col, val, z, ptr[row], ptr[row + 1], K, c, T(0)));
         });
     } else {
         constexpr int ROWS = ReduceTile<TPR>::kRows;
@@ -1145,7 +1147,7 @@ __global__ void __launch_bounds__(TPR == 1 ? grouped_threads<K>() : tile_threads
     double v = 0.0;
     if constexpr (TPR == 1) {
         v = run_tiles<K>(n, [&](int row, int) {
-            return step(row, strided_dot<T, 1>(col, val, x_cur, ptr[row], ptr[row + 1], K, c, T(0)));
+            return step(row, strided_dot<T, 1, T, K == 1>(col, val, x_cur, ptr[row], ptr[row + 1], K, c, T(0)));
         });
     } else {
         constexpr int ROWS = ReduceTile<TPR>::kRows;
