@@ -10,11 +10,11 @@
 //
 // Precision: g - c, r - c and W x (r - c) are taken in FP64 before they are rounded to FP32, which leaves less error near
 // a node than coordinates centred on the whole grid; both sums carry the same w. A block's sums over kStage nodes are
-// added to running sums of their own, so that rounding does not grow with the number of nodes.
+// added to running sums of their own, so that rounding does not grow with the number of nodes. The two sums of a node
+// cancel down to |g - r| / |g - c|, so a node nearer than an eighth of the tile's half diagonal keeps its own cross product.
 //
 // Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 47.7 ms against 73.7 for a cross product a pair
-// (26 operations a pair at the pipe's rate: 39 ms); 332k by 52k with one direction: 8.5 ms against 10.6. The largest error
-// against 64 bits 8.5e-6 of the largest value, 1.9e-5 before. The matrix w on the tensor cores (tcgen05 kind::tf32, w in two
+// (26 operations a pair at the pipe's rate: 39 ms); 332k by 52k with one direction: 8.5 ms against 10.6. The matrix w on the tensor cores (tcgen05 kind::tf32, w in two
 // terms from tensor memory, the weights in three) took 48.9 and 13.8 ms: a block there forms w, hands it over and waits in
 // step, and the pairs' distances alone, no matrix instruction issued, took 45.
 #include <algorithm>
@@ -30,6 +30,7 @@ constexpr int kPerThread = 4;                     // grid points a thread, as tw
 constexpr int kPoints = kThreads * kPerThread;    // points of a block's tile
 constexpr int kStage = 128;                       // nodes staged at once
 constexpr int kResident = 4;                      // blocks an SM
+constexpr double kNear = 8.0;                     // pairs within 1 / kNear of the tile's half diagonal are near
 
 // A staged node: -(r - c) and one unused word, then W and W x (r - c) of each direction.
 template <int ND>
@@ -80,9 +81,12 @@ __global__ void __launch_bounds__(kThreads, kResident)
     const int at[3] = {tile / (tiles.n[1] * tiles.n[2]) * tiles.t[0], tile / tiles.n[2] % tiles.n[1] * tiles.t[1],
                        tile % tiles.n[2] * tiles.t[2]};
     double center[3];
+    double lever2 = 0.0;  // |g - c|^2 of the tile's corners
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int extent = min(tiles.t[a], gr.shape[a] - at[a]);
+        const double half = gr.spacing_mm[a] * 0.5 * (extent - 1) * 1e-3;
+        lever2 += half * half;
         center[a] = (gr.origin_mm[a] + gr.spacing_mm[a] * (at[a] + 0.5 * (extent - 1))) * 1e-3;
     }
     // Point p of the tile: its place relative to the centre, and its index in the grid (-1 past the tile).
@@ -100,6 +104,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
         }
         return inside ? index : -1L;
     };
+    const float near2 = static_cast<float>(lever2 / (kNear * kNear));
     float2 gx[2], gy[2], gz[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -147,6 +152,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
             const float* r = rec + j * kWords;
             const float4 at4 = *reinterpret_cast<const float4*>(r);
             float wu[kPerThread];
+            float2 d2s[2];
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const float2 dx = __fadd2_rn(gx[q], make_float2(at4.x, at4.x));
@@ -155,10 +161,32 @@ __global__ void __launch_bounds__(kThreads, kResident)
                 float2 d2 = __fmul2_rn(dx, dx);
                 d2 = __ffma2_rn(dy, dy, d2);
                 d2 = __ffma2_rn(dz, dz, d2);
+                d2s[q] = d2;
                 const float2 inv = make_float2(rsqrt_fast(d2.x), rsqrt_fast(d2.y));
                 const float2 w = __fmul2_rn(__fmul2_rn(inv, inv), inv);
                 wu[2 * q] = w.x;
                 wu[2 * q + 1] = w.y;
+            }
+            // The split loses |g - c| / |g - r| in accuracy: a pair nearer than an eighth of the lever (a few nodes a
+            // point) takes its own cross product, straight into the running sums.
+            if (!(fminf(fminf(d2s[0].x, d2s[0].y), fminf(d2s[1].x, d2s[1].y)) >= near2)) {
+#pragma unroll
+                for (int u = 0; u < kPerThread; ++u) {
+                    const int q = u / 2;
+                    const float d2 = u % 2 ? d2s[q].y : d2s[q].x;
+                    if (d2 >= near2) continue;
+                    const float dx = (u % 2 ? gx[q].y : gx[q].x) + at4.x, dy = (u % 2 ? gy[q].y : gy[q].x) + at4.y;
+                    const float dz = (u % 2 ? gz[q].y : gz[q].x) + at4.z;
+#pragma unroll
+                    for (int d = 0; d < ND; ++d) {
+                        const float mx = r[4 + 6 * d], my = r[5 + 6 * d], mz = r[6 + 6 * d];
+                        float2* t = total + (u * kPairs + 3 * d) * kThreads + threadIdx.x;
+                        t[kThreads].y -= wu[u] * fmaf(my, dz, -mz * dy);
+                        t[2 * kThreads].x -= wu[u] * fmaf(mz, dx, -mx * dz);
+                        t[2 * kThreads].y -= wu[u] * fmaf(mx, dy, -my * dx);
+                    }
+                    wu[u] = 0.0f;
+                }
             }
 #pragma unroll
             for (int c = 0; c < kPairs; ++c) {

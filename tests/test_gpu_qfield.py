@@ -26,24 +26,34 @@ def adjoints(request):
     subj.free()
 
 
-@pytest.mark.parametrize("shape, spacing", [((1, 1, 1), (3, 3, 3)), ((1, 1, 40), (3, 3, 3)), ((8, 8, 8), (3, 3, 3)),
-                                           ((9, 8, 8), (2, 3, 4)), ((33, 2, 1), (5, 1, 1)), ((23, 17, 11), (3, 3, 3))])
-def test_field_against_the_sum_in_64_bits(adjoints, shape, spacing):
-    origin = np.array([-21.0, -19.5, 80.3])
-    sp = np.array(spacing, np.float64)
+def _check(adj, origin, sp, shape):
     grid = adm.Grid(origin_m=origin * 1e-3, spacing_m=sp * 1e-3, shape=shape)
     ijk = np.stack(np.meshgrid(*(np.arange(n) for n in shape), indexing="ij"), axis=-1).reshape(-1, 3)
     pts = (origin + ijk * sp) * 1e-3
     half = 0.5 * np.linalg.norm((np.array(shape) - 1) * sp) * 1e-3
+    q = adm.sample_qfield(adj, grid).q
+    w_all, nodes = adj.node_weights, adj.subject.context.array("nodes_mm").reshape(-1, 3) * 1e-3
+    assert q.shape == (len(w_all), *shape, 3)
+    for d, w in enumerate(w_all):
+        got = q[d].reshape(-1, 3).astype(np.float64)
+        for i in range(0, len(pts), 256):
+            diff = pts[i:i + 256, None] - nodes[None]
+            r = np.linalg.norm(diff, axis=2)
+            want = 1e-7 * (np.cross(w[None], diff) / r[..., None] ** 3).sum(1)
+            bound = 16 * 2.0**-24 * 1e-7 * ((r + 2 * half) * np.linalg.norm(w, axis=1) / r**3).sum(1)
+            assert (np.abs(got[i:i + 256] - want).max(1) <= bound).all()
+
+
+@pytest.mark.parametrize("gap_mm", [0.05, 0.6, 2.0])
+def test_a_point_beside_a_node(adjoints, gap_mm):
+    """Nodes nearer than an eighth of the tile's half diagonal take their own cross product."""
     for adj in adjoints:
-        q = adm.sample_qfield(adj, grid).q
-        w_all, nodes = adj.node_weights, adj.subject.context.array("nodes_mm").reshape(-1, 3) * 1e-3
-        assert q.shape == (len(w_all), *shape, 3)
-        for d, w in enumerate(w_all):
-            got = q[d].reshape(-1, 3).astype(np.float64)
-            for i in range(0, len(pts), 256):
-                diff = pts[i:i + 256, None] - nodes[None]
-                r = np.linalg.norm(diff, axis=2)
-                want = 1e-7 * (np.cross(w[None], diff) / r[..., None] ** 3).sum(1)
-                bound = 16 * 2.0**-24 * 1e-7 * ((r + 2 * half) * np.linalg.norm(w, axis=1) / r**3).sum(1)
-                assert (np.abs(got[i:i + 256] - want).max(1) <= bound).all()
+        node = adj.subject.context.array("nodes_mm").reshape(-1, 3)[-1]
+        _check(adj, node - [9.0, 12.0, 6.0] + [gap_mm, 0.0, 0.0], np.full(3, 3.0), (8, 8, 8))
+
+
+@pytest.mark.parametrize("shape, spacing", [((1, 1, 1), (3, 3, 3)), ((1, 1, 40), (3, 3, 3)), ((8, 8, 8), (3, 3, 3)),
+                                           ((9, 8, 8), (2, 3, 4)), ((33, 2, 1), (5, 1, 1)), ((23, 17, 11), (3, 3, 3))])
+def test_field_against_the_sum_in_64_bits(adjoints, shape, spacing):
+    for adj in adjoints:
+        _check(adj, np.array([-21.0, -19.5, 80.3]), np.array(spacing, np.float64), shape)
