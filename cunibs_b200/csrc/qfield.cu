@@ -13,10 +13,12 @@
 // added to running sums of their own, so that rounding does not grow with the number of nodes. The two sums of a node
 // cancel down to |g - r| / |g - c|, so a node nearer than an eighth of the tile's half diagonal keeps its own cross product.
 //
-// Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 47.7 ms against 73.7 for a cross product a pair
-// (26 operations a pair at the pipe's rate: 39 ms); 332k by 52k with one direction: 8.5 ms against 10.6. The matrix w on the tensor cores (tcgen05 kind::tf32, w in two
-// terms from tensor memory, the weights in three) took 48.9 and 13.8 ms: a block there forms w, hands it over and waits in
-// step, and the pairs' distances alone, no matrix instruction issued, took 45.
+// Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 47.7 ms before the near nodes' own products (26
+// operations a pair at the pipe's rate: 39 ms), about 3 more with them, against 73.7 for a cross product a pair; 332k by
+// 52k with one direction 8.5 (before the near nodes) against 10.6. The largest errors against 64 bits over two seeds'
+// grids 1.8e-6 and 5.7e-6, where a cross product a pair with grid-centred coordinates left 2.6e-5 and 1.8e-5. The matrix
+// w on the tensor cores (tcgen05 kind::tf32, w in two terms from tensor memory, the weights in three) took 48.9 and 13.8
+// ms: a block there forms w, hands it over and waits in step, and with one matrix instruction a chunk left it took 46.
 #include <algorithm>
 #include <cmath>
 
