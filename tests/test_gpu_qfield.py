@@ -8,8 +8,11 @@ a stage's nodes add their own few u: 16 u (|g - r| + 2 L) |W| / |g - r|^3 a pair
 
 from __future__ import annotations
 
+import time
+
 import numpy as np
 import pytest
+import torch
 
 from cunibs_b200 import Subject, adm
 from cunibs_b200.synthetic import sphere_head
@@ -57,3 +60,18 @@ def test_a_point_beside_a_node(adjoints, gap_mm):
 def test_field_against_the_sum_in_64_bits(adjoints, shape, spacing):
     for adj in adjoints:
         _check(adj, np.array([-21.0, -19.5, 80.3]), np.array(spacing, np.float64), shape)
+
+
+def test_sampling_is_over_when_the_call_returns(adjoints):
+    """A failure of the field's kernels is this call's, and its time too: next to nothing is left on the device."""
+    grid = adm.Grid(origin_m=np.array([-0.09, -0.09, 0.0]), spacing_m=np.full(3, 3e-3), shape=(60, 60, 60))
+    left = []
+    for _ in range(6):
+        torch.cuda.synchronize()
+        times = [time.perf_counter()]
+        adm.sample_qfield(adjoints[1], grid)
+        times.append(time.perf_counter())
+        torch.cuda.synchronize()
+        times.append(time.perf_counter())
+        left.append((times[2] - times[1]) / (times[2] - times[0]))
+    assert np.median(left[1:]) < 0.2
