@@ -8,17 +8,20 @@
 // reciprocal square root, where the cross product of every pair takes 8 + 9 n_dir. The products W x (r - c) are formed
 // once per block and node.
 //
-// Precision: g - c, r - c and W x (r - c) are taken in FP64 before they are rounded to FP32, which leaves less error near
-// a node than coordinates centred on the whole grid; both sums carry the same w. A block's sums over kStage nodes are
-// added to running sums of their own, so that rounding does not grow with the number of nodes. The two sums of a node
-// cancel down to |g - r| / |g - c|, so a node nearer than an eighth of the tile's half diagonal keeps its own cross product.
+// Precision: g - c, r - c and W x (r - c) are taken in FP64 before they are rounded to FP32; both sums carry the same w. A
+// block's sums over kStage nodes are added to running sums of their own, so that rounding does not grow with the number
+// of nodes. What the rounding of the places and the cancellation of the two sums cost grows as |g - c| / |g - r|, so the
+// nodes within 1 / kNear of the tile's half diagonal of its box take a cross product a point, with g - r and w from both
+// parts that FP32 makes of g - c and r - c. Relative to 64 bits over eleven grids of 3 mm (nodes 3 to 10 mm apart): 1.9e-7 to
+// 2.3e-7. A cross product a pair with grid-centred coordinates left 5.7e-7 to 1.2e-5; pairs nearer than an eighth of
+// the half diagonal kept apart, but with the rounded places, 4.3e-7 to 6.8e-6.
 //
-// Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 47.7 ms before the near nodes' own products (26
-// operations a pair at the pipe's rate: 39 ms), about 3 more with them, against 73.7 for a cross product a pair; 332k by
-// 52k with one direction 8.5 (before the near nodes) against 10.6. The largest errors against 64 bits over two seeds'
-// grids 1.8e-6 and 5.7e-6, where a cross product a pair with grid-centred coordinates left 2.6e-5 and 1.8e-5. The matrix
-// w on the tensor cores (tcgen05 kind::tf32, w in two terms from tensor memory, the weights in three) took 48.9 and 13.8
-// ms: a block there forms w, hands it over and waits in step, and with one matrix instruction a chunk left it took 46.
+// Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 49.6 ms (26 operations a pair at the pipe's
+// rate: 39 ms), one direction 28.6, against 73.7 and 35.0 for a cross product a pair and 50.6 and 29.8 with near pairs
+// tested for in the loop over the nodes: sorted apart while they are staged, the far ones need no test. The matrix
+// w on the tensor cores (tcgen05 kind::tf32, w in two terms from tensor memory, the weights in three) took 48.9 and,
+// for 332k points by 52k nodes and one direction, 13.8 ms, where this form took 47.7 and 8.5 before near nodes were
+// told apart: a block there forms w, hands it over and waits in step, and with one matrix instruction a chunk left it took 46.
 #include <algorithm>
 #include <cmath>
 
@@ -30,18 +33,23 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kPerThread = 4;                     // grid points a thread, as two pairs for the packed instructions
 constexpr int kPoints = kThreads * kPerThread;    // points of a block's tile
-constexpr int kStage = 128;                       // nodes staged at once
+constexpr int kStage = kThreads;                  // nodes staged at once, one a thread
 constexpr int kResident = 4;                      // blocks an SM
-constexpr double kNear = 8.0;                     // pairs within 1 / kNear of the tile's half diagonal are near
+// Nodes within 1 / kNear of the tile's half diagonal of its box are near: 8 leaves 2.6e-7 to 4.8e-7 on the 6 and 10 mm heads
+// with tiles of 8 x 8 x 8 and 3 x 15 x 11 points (restated on the CPU), 6 at most 3.0e-7 and 4 at most 3.6e-7, where a
+// dearer cross product takes twice the nodes (1.4% of a 179k-node head's for a tile in its middle).
+constexpr double kNear = 6.0;
 
-// A staged node: -(r - c) and one unused word, then W and W x (r - c) of each direction.
+// A staged node: -(r - c) and one unused word, then W and W x (r - c) of each direction; a near node holds the part
+// of -(r - c) that FP32 leaves in place of the first direction's W x (r - c).
 template <int ND>
 constexpr int record_words() {
     return (4 + 6 * ND + 3) / 4 * 4;
 }
+// The staged nodes, the running sums, and the part of the points' places that FP32 leaves.
 template <int ND>
 constexpr int smem_bytes() {
-    return static_cast<int>(sizeof(float)) * (kStage * record_words<ND>() + kPoints * 6 * ND);
+    return static_cast<int>(sizeof(float)) * (kStage * record_words<ND>() + kPoints * (6 * ND + 3));
 }
 
 __device__ __forceinline__ float rsqrt_fast(float x) {
@@ -78,21 +86,25 @@ __global__ void __launch_bounds__(kThreads, kResident)
                   float* __restrict__ out, float* __restrict__ part) {
     constexpr int kWords = record_words<ND>(), kPairs = 3 * ND;
     extern __shared__ __align__(16) float rec[];
+    __shared__ int far_in_warp[kThreads / 32];
     float2* total = reinterpret_cast<float2*>(rec + kStage * kWords);  // [point][pair of sums][thread]
+    float* low = reinterpret_cast<float*>(total + kPerThread * kPairs * kThreads);  // [axis][point][thread]
     const int tile = blockIdx.x % n_tiles, r0 = blockIdx.x / n_tiles;
     const int at[3] = {tile / (tiles.n[1] * tiles.n[2]) * tiles.t[0], tile / tiles.n[2] % tiles.n[1] * tiles.t[1],
                        tile % tiles.n[2] * tiles.t[2]};
     double center[3];
+    float half[3];        // of the tile's box
     double lever2 = 0.0;  // |g - c|^2 of the tile's corners
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const int extent = min(tiles.t[a], gr.shape[a] - at[a]);
-        const double half = gr.spacing_mm[a] * 0.5 * (extent - 1) * 1e-3;
-        lever2 += half * half;
+        const double h = gr.spacing_mm[a] * 0.5 * (extent - 1) * 1e-3;
+        half[a] = static_cast<float>(h);
+        lever2 += h * h;
         center[a] = (gr.origin_mm[a] + gr.spacing_mm[a] * (at[a] + 0.5 * (extent - 1))) * 1e-3;
     }
     // Point p of the tile: its place relative to the centre, and its index in the grid (-1 past the tile).
-    auto point = [&](int p, float (&g)[3]) {
+    auto point = [&](int p, double (&g)[3]) {
         const int in[3] = {p / (tiles.t[1] * tiles.t[2]), p / tiles.t[2] % tiles.t[1], p % tiles.t[2]};
         bool inside = p < tiles.t[0] * tiles.t[1] * tiles.t[2];
         long index = 0;
@@ -101,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
             const int extent = min(tiles.t[a], gr.shape[a] - at[a]);
             inside = inside && in[a] < extent;
             const int i = at[a] + min(in[a], extent - 1);
-            g[a] = static_cast<float>((gr.origin_mm[a] + gr.spacing_mm[a] * i) * 1e-3 - center[a]);
+            g[a] = (gr.origin_mm[a] + gr.spacing_mm[a] * i) * 1e-3 - center[a];
             index = index * gr.shape[a] + i;
         }
         return inside ? index : -1L;
@@ -109,32 +121,53 @@ __global__ void __launch_bounds__(kThreads, kResident)
     const float near2 = static_cast<float>(lever2 / (kNear * kNear));
     float2 gx[2], gy[2], gz[2];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        float g0[3], g1[3];
-        point(threadIdx.x + 2 * q * kThreads, g0);
-        point(threadIdx.x + (2 * q + 1) * kThreads, g1);
-        gx[q] = make_float2(g0[0], g1[0]);
-        gy[q] = make_float2(g0[1], g1[1]);
-        gz[q] = make_float2(g0[2], g1[2]);
+    for (int u = 0; u < kPerThread; ++u) {
+        double g[3];
+        point(threadIdx.x + u * kThreads, g);
+        const float h[3] = {static_cast<float>(g[0]), static_cast<float>(g[1]), static_cast<float>(g[2])};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) low[(a * kPerThread + u) * kThreads + threadIdx.x] = static_cast<float>(g[a] - h[a]);
+        (u % 2 ? gx[u / 2].y : gx[u / 2].x) = h[0];
+        (u % 2 ? gy[u / 2].y : gy[u / 2].x) = h[1];
+        (u % 2 ? gz[u / 2].y : gz[u / 2].x) = h[2];
     }
     for (int c = 0; c < kPerThread * kPairs; ++c) total[c * kThreads + threadIdx.x] = make_float2(0.f, 0.f);
     const int j_begin = r0 * run, j_end = min(n_src, j_begin + run);
     for (int j0 = j_begin; j0 < j_end; j0 += kStage) {
         const int nt = min(kStage, j_end - j0);
-        __syncthreads();
-        for (int j = threadIdx.x; j < nt; j += kThreads) {
-            float* r = rec + j * kWords;
-            double x[3];
+        // The far nodes go to the front of the stage, the near ones to its end.
+        const int j = j0 + threadIdx.x;
+        double x[3];
+        float hi[3], box2 = 0.0f;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                x[a] = src[static_cast<long>(a) * n_src + j0 + j] - center[a];
-                r[a] = -static_cast<float>(x[a]);
-            }
+        for (int a = 0; a < 3; ++a) {
+            x[a] = threadIdx.x < nt ? src[static_cast<long>(a) * n_src + j] - center[a] : 0.0;
+            hi[a] = static_cast<float>(x[a]);
+            const float past = fmaxf(fabsf(hi[a]) - half[a], 0.0f);
+            box2 = fmaf(past, past, box2);
+        }
+        const bool is_near = box2 < near2;
+        const unsigned staged = __ballot_sync(0xffffffffu, threadIdx.x < nt);
+        const unsigned far = __ballot_sync(0xffffffffu, threadIdx.x < nt && !is_near);
+        if (threadIdx.x % 32 == 0) far_in_warp[threadIdx.x / 32] = __popc(far);
+        __syncthreads();
+        int n_far = 0, far_before = 0;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) {
+            if (w < threadIdx.x / 32) far_before += far_in_warp[w];
+            n_far += far_in_warp[w];
+        }
+        if (threadIdx.x < nt) {
+            const unsigned below = (1u << threadIdx.x % 32) - 1;
+            const int near_before = threadIdx.x / 32 * 32 - far_before + __popc(staged & ~far & below);
+            float* r = rec + (is_near ? n_far + near_before : far_before + __popc(far & below)) * kWords;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) r[a] = -hi[a];
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
                 double m[3];
 #pragma unroll
-                for (int a = 0; a < 3; ++a) m[a] = src[(3L + 3 * d + a) * n_src + j0 + j];
+                for (int a = 0; a < 3; ++a) m[a] = src[(3L + 3 * d + a) * n_src + j];
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     const int u = (a + 1) % 3, v = (a + 2) % 3;
@@ -142,6 +175,9 @@ __global__ void __launch_bounds__(kThreads, kResident)
                     r[7 + 6 * d + a] = static_cast<float>(m[u] * x[v] - m[v] * x[u]);
                 }
             }
+            if (is_near)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) r[7 + a] = static_cast<float>(hi[a] - x[a]);
         }
         __syncthreads();
         float2 acc[kPerThread][kPairs];
@@ -150,11 +186,10 @@ __global__ void __launch_bounds__(kThreads, kResident)
 #pragma unroll
             for (int c = 0; c < kPairs; ++c) acc[u][c] = make_float2(0.f, 0.f);
 #pragma unroll 1
-        for (int j = 0; j < nt; ++j) {
-            const float* r = rec + j * kWords;
+        for (int i = 0; i < n_far; ++i) {
+            const float* r = rec + i * kWords;
             const float4 at4 = *reinterpret_cast<const float4*>(r);
             float wu[kPerThread];
-            float2 d2s[2];
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const float2 dx = __fadd2_rn(gx[q], make_float2(at4.x, at4.x));
@@ -163,38 +198,38 @@ __global__ void __launch_bounds__(kThreads, kResident)
                 float2 d2 = __fmul2_rn(dx, dx);
                 d2 = __ffma2_rn(dy, dy, d2);
                 d2 = __ffma2_rn(dz, dz, d2);
-                d2s[q] = d2;
                 const float2 inv = make_float2(rsqrt_fast(d2.x), rsqrt_fast(d2.y));
                 const float2 w = __fmul2_rn(__fmul2_rn(inv, inv), inv);
                 wu[2 * q] = w.x;
                 wu[2 * q + 1] = w.y;
-            }
-            // The split loses |g - c| / |g - r| in accuracy: a pair nearer than an eighth of the lever (a few nodes a
-            // point) takes its own cross product, straight into the running sums.
-            if (!(fminf(fminf(d2s[0].x, d2s[0].y), fminf(d2s[1].x, d2s[1].y)) >= near2)) {
-#pragma unroll
-                for (int u = 0; u < kPerThread; ++u) {
-                    const int q = u / 2;
-                    const float d2 = u % 2 ? d2s[q].y : d2s[q].x;
-                    if (d2 >= near2) continue;
-                    const float dx = (u % 2 ? gx[q].y : gx[q].x) + at4.x, dy = (u % 2 ? gy[q].y : gy[q].x) + at4.y;
-                    const float dz = (u % 2 ? gz[q].y : gz[q].x) + at4.z;
-#pragma unroll
-                    for (int d = 0; d < ND; ++d) {
-                        const float mx = r[4 + 6 * d], my = r[5 + 6 * d], mz = r[6 + 6 * d];
-                        float2* t = total + (u * kPairs + 3 * d) * kThreads + threadIdx.x;
-                        t[kThreads].y -= wu[u] * fmaf(my, dz, -mz * dy);
-                        t[2 * kThreads].x -= wu[u] * fmaf(mz, dx, -mx * dz);
-                        t[2 * kThreads].y -= wu[u] * fmaf(mx, dy, -my * dx);
-                    }
-                    wu[u] = 0.0f;
-                }
             }
 #pragma unroll
             for (int c = 0; c < kPairs; ++c) {
                 const float2 m = *reinterpret_cast<const float2*>(r + 4 + 2 * c);
 #pragma unroll
                 for (int u = 0; u < kPerThread; ++u) acc[u][c] = __ffma2_rn(make_float2(wu[u], wu[u]), m, acc[u][c]);
+            }
+        }
+        // The near nodes: g - r to FP32's last place from both parts, and the cross product itself, into the second sum.
+#pragma unroll 1
+        for (int i = n_far; i < nt; ++i) {
+            const float* r = rec + i * kWords;
+#pragma unroll
+            for (int u = 0; u < kPerThread; ++u) {
+                const float* lo = low + u * kThreads + threadIdx.x;
+                const float dx = ((u % 2 ? gx[u / 2].y : gx[u / 2].x) + r[0]) + (lo[0] + r[7]);
+                const float dy = ((u % 2 ? gy[u / 2].y : gy[u / 2].x) + r[1]) + (lo[kPoints] + r[8]);
+                const float dz = ((u % 2 ? gz[u / 2].y : gz[u / 2].x) + r[2]) + (lo[2 * kPoints] + r[9]);
+                const float inv = rsqrt_fast(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+                const float w = -(inv * inv * inv);
+#pragma unroll
+                for (int d = 0; d < ND; ++d) {
+                    const float mx = r[4 + 6 * d], my = r[5 + 6 * d], mz = r[6 + 6 * d];
+                    float2* t = &acc[u][3 * d];
+                    t[1].y = fmaf(w, fmaf(my, dz, -mz * dy), t[1].y);
+                    t[2].x = fmaf(w, fmaf(mz, dx, -mx * dz), t[2].x);
+                    t[2].y = fmaf(w, fmaf(mx, dy, -my * dx), t[2].y);
+                }
             }
         }
 #pragma unroll
@@ -210,9 +245,10 @@ __global__ void __launch_bounds__(kThreads, kResident)
     const float sc = part ? 1.0f : scale;
 #pragma unroll 1
     for (int u = 0; u < kPerThread; ++u) {
-        float g[3];
-        const long index = point(threadIdx.x + u * kThreads, g);
+        double gd[3];
+        const long index = point(threadIdx.x + u * kThreads, gd);
         if (index < 0) continue;
+        const float g[3] = {static_cast<float>(gd[0]), static_cast<float>(gd[1]), static_cast<float>(gd[2])};
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
             const float2* t = total + (u * kPairs + 3 * d) * kThreads + threadIdx.x;
