@@ -1419,7 +1419,7 @@ int cunibs_adm_sample(cunibs_adm* a, const double* origin_mm, const double* spac
         a->Q.resize(3 * static_cast<std::size_t>(n_grid) * a->dirs.n);
         // Q_d on the grid: the coil-field N-body with the mesh nodes as sources (reciprocity.py:183-213).
         qfield_sample(a->ctx->mesh, gr, a->W.get(), a->dirs.n, a->Q.get(), a->q_sources, a->q_part,
-                      a->ctx->sm_count, s);
+                      a->ctx->sm_count, 1e3 * a->ctx->mesh_rho_m, s);
         CUNIBS_CHECK(cudaStreamSynchronize(s));  // a handle marked sampled holds its field
         a->grid = gr;
         a->sampled = true;

@@ -468,11 +468,11 @@ void adm_node_weights(const Mesh& m, const double* lam, int K, const double* alp
                       double* W, cudaStream_t s);
 void adm_centred_nodes(const Mesh& m, const double* center_mm, double* out_m, cudaStream_t s);
 // The reciprocity field Q (n_dir, n_grid, 3) of the nodal weights W (n_dir, n_nodes, 3) on a grid, every
-// direction in one pass over the sources (qfield.cu). sources holds them by axis, scratch the source runs' partial fields when
-// the grid alone does not fill the GPU (grown on demand and kept by the caller, so repeated calls
-// allocate nothing).
+// direction in one pass over the sources (qfield.cu). reach_mm: the mesh's farthest node from its middle. sources holds the
+// nodes by axis, scratch the source runs' partial fields when the grid alone does not fill the GPU (grown on demand and kept
+// by the caller, so repeated calls allocate nothing).
 void qfield_sample(const Mesh& m, const AdmGrid& gr, const double* W, int n_dir, float* Q, DevArray<double>& sources,
-                   DevArray<float>& scratch, int sm_count, cudaStream_t s);
+                   DevArray<float>& scratch, int sm_count, double reach_mm, cudaStream_t s);
 // E (P, n_dir) from the sampled field Q (n_dir, n_grid, 3); bad[3] receives, per axis, the smallest
 // flat sample index p * n_dip + j of a dipole off the grid (left untouched when none is).
 void adm_evaluate(const float* Q, int n_dir, const AdmGrid& gr, const double* pos, const double* mom, int n_dip,

@@ -12,12 +12,12 @@
 // block's sums over kStage nodes are added to running sums of their own, so that rounding does not grow with the number
 // of nodes. What the rounding of the places and the cancellation of the two sums cost grows as |g - c| / |g - r|, so the
 // nodes within 1 / kNear of the tile's half diagonal of its box take a cross product a point, with g - r and w from both
-// parts that FP32 makes of g - c and r - c. Relative to 64 bits over eleven grids of 3 mm (nodes 3 to 10 mm apart): 1.9e-7 to
-// 2.3e-7. A cross product a pair with grid-centred coordinates left 5.7e-7 to 1.2e-5; pairs nearer than an eighth of
+// parts that FP32 makes of g - c and r - c. Relative to 64 bits over eleven grids of 3 mm (nodes 3 to 10 mm apart): 1.8e-7 to
+// 2.2e-7. A cross product a pair with grid-centred coordinates left 5.7e-7 to 1.2e-5; pairs nearer than an eighth of
 // the half diagonal kept apart, but with the rounded places, 4.3e-7 to 6.8e-6.
 //
-// Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 49.6 ms (26 operations a pair at the pipe's
-// rate: 39 ms), one direction 28.6, against 73.7 and 35.0 for a cross product a pair and 50.6 and 29.8 with near pairs
+// Bound: the FP32 pipe. 301k points by 179k nodes with three directions: 49.8 ms (26 operations a pair at the pipe's
+// rate: 39 ms), one direction 28.9, against 73.7 and 35.0 for a cross product a pair and 50.6 and 29.8 with near pairs
 // tested for in the loop over the nodes: sorted apart while they are staged, the far ones need no test. The matrix
 // w on the tensor cores (tcgen05 kind::tf32, w in two terms from tensor memory, the weights in three) took 48.9 and,
 // for 332k points by 52k nodes and one direction, 13.8 ms, where this form took 47.7 and 8.5 before near nodes were
@@ -34,6 +34,7 @@ constexpr int kThreads = 128;
 constexpr int kPerThread = 4;                     // grid points a thread, as two pairs for the packed instructions
 constexpr int kPoints = kThreads * kPerThread;    // points of a block's tile
 constexpr int kStage = kThreads;                  // nodes staged at once, one a thread
+constexpr int kMaxGroups = 16;                    // groups of threads that share a small tile's nodes
 constexpr int kResident = 4;                      // blocks an SM
 // Nodes within 1 / kNear of the tile's half diagonal of its box are near: 8 leaves 2.6e-7 to 4.8e-7 on the 6 and 10 mm heads
 // with tiles of 8 x 8 x 8 and 3 x 15 x 11 points (restated on the CPU), 6 at most 3.0e-7 and 4 at most 3.6e-7, where a
@@ -58,10 +59,11 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
     return r;
 }
 
-// Boxes of t[0] x t[1] x t[2] <= kPoints grid points; n[a] of them along axis a.
+// Boxes of t[0] x t[1] x t[2] <= kPoints / groups grid points; n[a] of them along axis a.
 struct QTiles {
     int t[3];
     int n[3];
+    int groups;
 };
 
 // Sources as the kernel reads them, one array per axis: positions in metres (3, n), then the weights of each
@@ -79,8 +81,9 @@ __global__ void sources_kernel(const double* __restrict__ nodes_mm, const double
 // Work item = (tile of grid points, run of sources): item = run * n_tiles + tile. With one run the scaled
 // field goes to out; with several the run's unscaled partial goes to part[run], and partial_sum_kernel
 // adds the runs in order. The runs depend on the sizes only, never on ND, and a direction's sums are the same
-// operations whatever ND.
-template <int ND>
+// operations whatever ND. A tile of at most half the block's points (GROUPED) is held by 2 to 16 groups of
+// threads, each with every point and its share of the staged nodes; their sums are added in order at the end.
+template <int ND, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, kResident)
     qfield_kernel(AdmGrid gr, QTiles tiles, int n_tiles, const double* __restrict__ src, int n_src, int run, float scale,
                   float* __restrict__ out, float* __restrict__ part) {
@@ -89,6 +92,9 @@ __global__ void __launch_bounds__(kThreads, kResident)
     __shared__ int far_in_warp[kThreads / 32];
     float2* total = reinterpret_cast<float2*>(rec + kStage * kWords);  // [point][pair of sums][thread]
     float* low = reinterpret_cast<float*>(total + kPerThread * kPairs * kThreads);  // [axis][point][thread]
+    const int groups = GROUPED ? tiles.groups : 1;
+    const int width = kThreads / groups;  // threads a group
+    const int group = GROUPED ? threadIdx.x / width : 0, lane = GROUPED ? threadIdx.x % width : threadIdx.x;
     const int tile = blockIdx.x % n_tiles, r0 = blockIdx.x / n_tiles;
     const int at[3] = {tile / (tiles.n[1] * tiles.n[2]) * tiles.t[0], tile / tiles.n[2] % tiles.n[1] * tiles.t[1],
                        tile % tiles.n[2] * tiles.t[2]};
@@ -123,7 +129,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
 #pragma unroll
     for (int u = 0; u < kPerThread; ++u) {
         double g[3];
-        point(threadIdx.x + u * kThreads, g);
+        point(lane + u * width, g);
         const float h[3] = {static_cast<float>(g[0]), static_cast<float>(g[1]), static_cast<float>(g[2])};
 #pragma unroll
         for (int a = 0; a < 3; ++a) low[(a * kPerThread + u) * kThreads + threadIdx.x] = static_cast<float>(g[a] - h[a]);
@@ -133,6 +139,8 @@ __global__ void __launch_bounds__(kThreads, kResident)
     }
     for (int c = 0; c < kPerThread * kPairs; ++c) total[c * kThreads + threadIdx.x] = make_float2(0.f, 0.f);
     const int j_begin = r0 * run, j_end = min(n_src, j_begin + run);
+    float2 acc[kPerThread][kPairs];
+    int turn = 0;  // stages since the sums in acc began
     for (int j0 = j_begin; j0 < j_end; j0 += kStage) {
         const int nt = min(kStage, j_end - j0);
         // The far nodes go to the front of the stage, the near ones to its end.
@@ -180,13 +188,14 @@ __global__ void __launch_bounds__(kThreads, kResident)
                 for (int a = 0; a < 3; ++a) r[7 + a] = static_cast<float>(hi[a] - x[a]);
         }
         __syncthreads();
-        float2 acc[kPerThread][kPairs];
+        if (turn == 0) {
 #pragma unroll
-        for (int u = 0; u < kPerThread; ++u)
+            for (int u = 0; u < kPerThread; ++u)
 #pragma unroll
-            for (int c = 0; c < kPairs; ++c) acc[u][c] = make_float2(0.f, 0.f);
+                for (int c = 0; c < kPairs; ++c) acc[u][c] = make_float2(0.f, 0.f);
+        }
 #pragma unroll 1
-        for (int i = 0; i < n_far; ++i) {
+        for (int i = group; i < n_far; i += groups) {
             const float* r = rec + i * kWords;
             const float4 at4 = *reinterpret_cast<const float4*>(r);
             float wu[kPerThread];
@@ -212,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, kResident)
         }
         // The near nodes: g - r to FP32's last place from both parts, and the cross product itself, into the second sum.
 #pragma unroll 1
-        for (int i = n_far; i < nt; ++i) {
+        for (int i = n_far + group; i < nt; i += groups) {
             const float* r = rec + i * kWords;
 #pragma unroll
             for (int u = 0; u < kPerThread; ++u) {
@@ -232,27 +241,37 @@ __global__ void __launch_bounds__(kThreads, kResident)
                 }
             }
         }
+        if (++turn == groups || j0 + kStage >= j_end) {
+            turn = 0;
 #pragma unroll
-        for (int u = 0; u < kPerThread; ++u)
+            for (int u = 0; u < kPerThread; ++u)
 #pragma unroll
-            for (int c = 0; c < kPairs; ++c) {
-                float2* t = total + (u * kPairs + c) * kThreads + threadIdx.x;
-                *t = __fadd2_rn(*t, acc[u][c]);
-            }
+                for (int c = 0; c < kPairs; ++c) {
+                    float2* t = total + (u * kPairs + c) * kThreads + threadIdx.x;
+                    *t = __fadd2_rn(*t, acc[u][c]);
+                }
+        }
     }
+    if (GROUPED) __syncthreads();
     const long count = static_cast<long>(gr.shape[0]) * gr.shape[1] * gr.shape[2];
     float* o = part ? part + static_cast<long>(r0) * ND * count * 3 : out;
     const float sc = part ? 1.0f : scale;
 #pragma unroll 1
-    for (int u = 0; u < kPerThread; ++u) {
+    for (int p = threadIdx.x; p < kPerThread * width; p += kThreads) {
         double gd[3];
-        const long index = point(threadIdx.x + u * kThreads, gd);
+        const long index = point(p, gd);
         if (index < 0) continue;
         const float g[3] = {static_cast<float>(gd[0]), static_cast<float>(gd[1]), static_cast<float>(gd[2])};
+        const int u = p / width;
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
-            const float2* t = total + (u * kPairs + 3 * d) * kThreads + threadIdx.x;
-            const float2 t0 = t[0], t1 = t[kThreads], t2 = t[2 * kThreads];
+            const float2* t = total + (u * kPairs + 3 * d) * kThreads + p % width;
+            float2 t0 = t[0], t1 = t[kThreads], t2 = t[2 * kThreads];
+            for (int h = 1; h < groups; ++h) {
+                t0 = __fadd2_rn(t0, t[h * width]);
+                t1 = __fadd2_rn(t1, t[kThreads + h * width]);
+                t2 = __fadd2_rn(t2, t[2 * kThreads + h * width]);
+            }
             const float m[3] = {t0.x, t0.y, t1.x}, w[3] = {t1.y, t2.x, t2.y};
             float* q = o + (static_cast<long>(d) * count + index) * 3;
             q[0] = sc * (fmaf(m[1], g[2], -m[2] * g[1]) - w[0]);
@@ -268,77 +287,105 @@ __global__ void partial_sum_kernel(long count, int runs, const float* __restrict
     const long q = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= count) return;
     float v = part[q];
+#pragma unroll 8
     for (int c = 1; c < runs; ++c) v += part[c * count + q];
     out[q] = scale * v;
 }
 
-// The box of at most kPoints points that covers the grid with the fewest tiles, compact first on ties
-// (the lever arm |g - c| multiplies the sums' rounding): sides up to 32, the longest at most four times the
-// shortest side that is not the whole axis.
-QTiles choose_tiles(const AdmGrid& gr) {
+// The tiles that cover the grid at the least cost: per tile a stage's nodes over the groups that share them
+// (with the staging worth kStageNodes more), and the near nodes kNearCost dearer (they take 14 + 9 n_dir operations a
+// pair), where they are the share that the box and its near shell have of a ball of the mesh's reach. So a thick grid takes
+// compact full tiles, a plane full tiles of one layer, and a line or a handful of points a few points held by many groups.
+// One direction by 179k nodes, in ms: boxes near a cube's diagonal by one group and at most 16 runs; this rule; a cross
+// product for every pair over the points in order:
+//     200 x 200 points 9.78, 4.42, 4.75;    4096 in a line 6.31, 0.55, 0.56;    10^3 0.94, 0.18, 0.22;
+//     16^3 0.94, 0.48, 0.56;    74 x 74 x 55 28.6, 28.9, 35.0.
+// At 20 mm between points near shells take most of the head: 60^3 points by 121k nodes 15.2 ms, three directions 26.1 (25.3
+// with the pairs tested one by one, 36.5 with a cross product for every pair).
+constexpr double kStageNodes = 4.0;
+constexpr double kNearCost = 1.0;
+constexpr int kMaxSide = 64;
+
+QTiles choose_tiles(const AdmGrid& gr, double reach_mm) {
     QTiles best{};
     double best_cost = INFINITY;
-    for (int x = 1; x <= 32; ++x)
-        for (int y = 1; y <= 32; ++y) {
-            if (x * y > kPoints) break;
-            const int z = std::min(32, kPoints / (x * y));
-            const int t[3] = {std::min(x, gr.shape[0]), std::min(y, gr.shape[1]), std::min(z, gr.shape[2])};
-            double n = 1.0, lever = 0.0;
-            for (int a = 0; a < 3; ++a) {
-                n *= (gr.shape[a] + t[a] - 1) / t[a];
-                lever += (t[a] * gr.spacing_mm[a]) * (t[a] * gr.spacing_mm[a]);
-            }
-            const double cube = 3.0 * std::pow(kPoints * gr.spacing_mm[0] * gr.spacing_mm[1] * gr.spacing_mm[2], 2.0 / 3.0);
-            if (lever > 2.25 * cube && x * y * z > 1 && best_cost < INFINITY) continue;  // at most 1.5 times a cube's diagonal
-            const double cost = n * (1.0 + 0.02 * lever / cube);
-            if (cost < best_cost) {
+    const double ball = 4.18879 * reach_mm * reach_mm * reach_mm;
+    for (int groups = 1; groups <= kMaxGroups; groups *= 2) {
+        const int points = kPoints / groups;
+        const double stage = static_cast<double>(kStage) / groups + kStageNodes;
+        for (int x = 1; x <= std::min({points, kMaxSide, gr.shape[0]}); ++x)
+            for (int y = 1; y <= std::min({points / x, kMaxSide, gr.shape[1]}); ++y) {
+                const int t[3] = {x, y, std::min({points / (x * y), kMaxSide, gr.shape[2]})};
+                double cost = stage;
+                for (int a = 0; a < 3; ++a) cost *= (gr.shape[a] + t[a] - 1) / t[a];
+                if (cost >= best_cost) continue;
+                double side[3], lever2 = 0.0, box = 1.0;
+                for (int a = 0; a < 3; ++a) {
+                    side[a] = gr.spacing_mm[a] * (t[a] - 1);
+                    lever2 += 0.25 * side[a] * side[a];
+                }
+                const double shell = 2.0 * std::sqrt(lever2) / kNear;
+                for (int a = 0; a < 3; ++a) box *= side[a] + shell;
+                cost *= 1.0 + kNearCost * std::min(1.0, box / ball);
+                if (cost >= best_cost) continue;
                 best_cost = cost;
+                best.groups = groups;
                 for (int a = 0; a < 3; ++a) best.t[a] = t[a];
             }
-        }
+    }
     for (int a = 0; a < 3; ++a) best.n[a] = (gr.shape[a] + best.t[a] - 1) / best.t[a];
     return best;
+}
+
+// Nodes of a run: the fewest runs of sources whose waves of blocks (kResident per SM) take within 2% of the least time, a
+// run's partial field counted with the nodes whose time it takes to write and to add.
+int choose_run(int n_tiles, double points, int n_nodes, int slots) {
+    const int stages = (n_nodes + kStage - 1) / kStage;
+    const int most = std::min(stages, std::max(16, slots / n_tiles));
+    const double partial = 0.5 + points / 4e4;
+    auto cost = [&](int runs) {
+        const int each = (stages + runs - 1) / runs;
+        const double blocks = static_cast<double>(n_tiles) * ((stages + each - 1) / each);
+        return std::ceil(blocks / slots) * each * kStage + (runs > 1 ? runs * partial : 0.0);
+    };
+    double least = INFINITY;
+    for (int runs = 1; runs <= most; ++runs) least = std::min(least, cost(runs));
+    int runs = 1;
+    while (cost(runs) > 1.02 * least) ++runs;
+    return (stages + runs - 1) / runs * kStage;
 }
 
 }  // namespace
 
 void qfield_sample(const Mesh& m, const AdmGrid& gr, const double* W, int n_dir, float* Q, DevArray<double>& sources,
-                   DevArray<float>& scratch, int sm_count, cudaStream_t s) {
+                   DevArray<float>& scratch, int sm_count, double reach_mm, cudaStream_t s) {
     if (n_dir < 1 || n_dir > kAdmMaxDir) fail(kEInval, "between 1 and 3 adjoint directions");
     sources.reserve(3 * static_cast<std::size_t>(m.n_nodes) * (1 + n_dir));
     sources_kernel<<<grid_for(m.n_nodes), kBlock, 0, s>>>(m.nodes.get(), W, m.n_nodes, n_dir, sources.get());
     count_launch();
-    const QTiles tiles = choose_tiles(gr);
+    const QTiles tiles = choose_tiles(gr, reach_mm);
     const int n_tiles = tiles.n[0] * tiles.n[1] * tiles.n[2];
-    // Runs of sources so that the last wave of blocks (kResident per SM) is nearly full: the fewest that reach
-    // 97% of whole waves, else the best of 16; a run holds at least 1024 sources.
-    const int slots = sm_count * kResident;
-    int runs = 1;
-    double best = 0.0;
-    for (int c = 1; c <= std::max(1, std::min(16, m.n_nodes / 1024)); ++c) {
-        const double items = static_cast<double>(n_tiles) * c;
-        const double full = items / (std::ceil(items / slots) * slots);
-        if (full > best + 1e-9) {
-            best = full;
-            runs = c;
-        }
-        if (full >= 0.97) break;
-    }
-    const int run = ((m.n_nodes + runs - 1) / runs + kStage - 1) / kStage * kStage;
-    runs = (m.n_nodes + run - 1) / run;
+    const double points = static_cast<double>(gr.shape[0]) * gr.shape[1] * gr.shape[2];
+    const int run = choose_run(n_tiles, points, m.n_nodes, sm_count * kResident);
+    const int runs = (m.n_nodes + run - 1) / run;
     const long count = static_cast<long>(gr.shape[0]) * gr.shape[1] * gr.shape[2] * 3 * n_dir;
     if (runs > 1) scratch.reserve(static_cast<std::size_t>(count) * runs);
     float* part = runs > 1 ? scratch.get() : nullptr;
-    auto go = [&](auto nd) {
+    auto go = [&](auto nd, auto grouped) {
         constexpr int ND = decltype(nd)::value;
-        CUNIBS_CHECK(cudaFuncSetAttribute(qfield_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<ND>()));
-        qfield_kernel<ND><<<n_tiles * runs, kThreads, smem_bytes<ND>(), s>>>(gr, tiles, n_tiles, sources.get(), m.n_nodes,
-                                                                             run, 1e-7f, Q, part);
+        const auto kernel = qfield_kernel<ND, decltype(grouped)::value>;
+        CUNIBS_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<ND>()));
+        kernel<<<n_tiles * runs, kThreads, smem_bytes<ND>(), s>>>(gr, tiles, n_tiles, sources.get(), m.n_nodes, run, 1e-7f,
+                                                                  Q, part);
         count_launch();
     };
-    if (n_dir == 1) go(std::integral_constant<int, 1>{});
-    else if (n_dir == 2) go(std::integral_constant<int, 2>{});
-    else go(std::integral_constant<int, 3>{});
+    auto pick = [&](auto nd) {
+        if (tiles.groups > 1) go(nd, std::true_type{});
+        else go(nd, std::false_type{});
+    };
+    if (n_dir == 1) pick(std::integral_constant<int, 1>{});
+    else if (n_dir == 2) pick(std::integral_constant<int, 2>{});
+    else pick(std::integral_constant<int, 3>{});
     CUNIBS_LAUNCH_CHECK("reciprocity field");
     if (runs > 1) {
         partial_sum_kernel<<<grid_for(count), kBlock, 0, s>>>(count, runs, part, 1e-7f, Q);

@@ -1,5 +1,5 @@
-"""The reciprocity field's kernel at grids around its tiles of 512 points and node counts around its stages of
-128 nodes and runs of 1024, one to three directions, against the sum in FP64. Needs a B200.
+"""The reciprocity field's kernel at grids around its tiles of 512 points, smaller tiles held by 2 to 16 groups of
+threads, and node counts around its stages of 128 nodes, one to three directions, against the sum in FP64. Needs a B200.
 
 Each operation rounds in FP32 (u = 2^-24). A pair's places are off by u (|g - c| + |r - c|) from the tile's centre c, which
 changes 1/|g - r|^3 by three times that over |g - r|; its two sums cancel down to |g - r| from terms of the size of
@@ -64,8 +64,10 @@ def test_a_point_beside_a_node(adjoints, gap_mm, corner):
 
 
 @pytest.mark.parametrize("shape, spacing, tile", [
-    ((1, 1, 1), (3, 3, 3), (1, 1, 1)), ((1, 1, 40), (3, 3, 3), (1, 1, 20)), ((8, 8, 8), (3, 3, 3), (8, 8, 8)),
-    ((9, 8, 8), (2, 3, 4), (9, 8, 8)), ((33, 2, 1), (5, 1, 1), (33, 2, 1)), ((23, 17, 11), (3, 3, 3), (5, 9, 11))])
+    ((1, 1, 1), (3, 3, 3), (1, 1, 1)), ((1, 1, 40), (3, 3, 3), (1, 1, 40)), ((1, 1, 200), (3, 3, 3), (1, 1, 32)),
+    ((5, 5, 5), (3, 3, 3), (5, 5, 5)), ((6, 6, 6), (3, 3, 3), (6, 6, 6)), ((3, 3, 100), (3, 3, 3), (3, 3, 28)),
+    ((8, 8, 8), (3, 3, 3), (8, 8, 8)), ((9, 8, 8), (2, 3, 4), (1, 8, 8)), ((12, 9, 10), (20, 20, 20), (4, 3, 5)),
+    ((33, 2, 1), (5, 1, 1), (11, 2, 1)), ((70, 66, 1), (1, 1, 1), (14, 33, 1)), ((23, 17, 11), (3, 3, 3), (23, 1, 11))])
 def test_field_against_the_sum_in_64_bits(adjoints, shape, spacing, tile):
     for adj in adjoints:
         _check(adj, np.array([-21.0, -19.5, 80.3]), np.array(spacing, np.float64), shape, tile)
@@ -84,3 +86,27 @@ def test_sampling_is_over_when_the_call_returns(adjoints):
         times.append(time.perf_counter())
         left.append((times[2] - times[1]) / (times[2] - times[0]))
     assert np.median(left[1:]) < 0.2
+
+
+def _ms_a_point(adj, shape):
+    grid = adm.Grid(origin_m=np.array([0.0, 0.0, 75.0]) * 1e-3 - 1.5e-3 * (np.array(shape) - 1), spacing_m=np.full(3, 3e-3),
+                    shape=shape)
+    times = []
+    for _ in range(7):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        adm.sample_qfield(adj, grid)
+        torch.cuda.synchronize()
+        times.append(time.perf_counter() - t)
+    return 1e3 * np.median(times[2:]) / grid.n_points
+
+
+def test_flat_and_small_grids_cost_what_their_points_do():
+    """A point of a plane, a line or a small box costs little more than one of a thick box: 1.15, 1.41 and 1.22 times on 179k
+    nodes, where compact boxes and at most 16 runs of nodes for all of them took 2.6, 16 and 2.4 times."""
+    with Subject(sphere_head(4.0, 90.0, jitter_mm=0.2, seed=4), tolerance=1e-6) as subj:
+        adj = adm.solve_adjoint(subj, adm.resolve_target(subj, adm.Target([0.0, 0.0, 62.0], (0.0, 1.0, 0.0))), tolerance=1e-6)
+        thick = _ms_a_point(adj, (60, 60, 60))
+        assert _ms_a_point(adj, (200, 200, 1)) < 1.8 * thick
+        assert _ms_a_point(adj, (1, 1, 16384)) < 2.0 * thick
+        assert _ms_a_point(adj, (16, 16, 16)) < 2.5 * thick
