@@ -6,7 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
-#include <map>
+#include <numeric>
 #include <string>
 #include <type_traits>
 
@@ -1310,18 +1310,29 @@ int cunibs_adm_create(cunibs_context* c, const int* elem_idx, const double* weig
         require(!c->study, "a conductivity study is open: end it first");
         require(c->pending.empty(), "finish the submitted blocks first");
         Mesh& m = c->mesh;
-        std::map<int, double> target;  // an element named twice has both weights
+        bool ascending = true;  // and distinct, as a resolved target's are
         for (int i = 0; i < n_elem; ++i) {
             require(elem_idx[i] >= 0 && elem_idx[i] < m.n_tets, "target element index out of range");
             require(std::isfinite(weights[i]), "target weights must be finite");
-            target[elem_idx[i]] += weights[i];
+            ascending = ascending && (i == 0 || elem_idx[i] > elem_idx[i - 1]);
         }
         std::vector<int> t_idx;
         std::vector<double> t_w;
-        for (const auto& t : target) {
-            t_idx.push_back(t.first);
-            t_w.push_back(t.second);
+        if (!ascending) {  // an element named twice has both weights, added in the order given
+            std::vector<int> order(n_elem);
+            std::iota(order.begin(), order.end(), 0);
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return elem_idx[x] < elem_idx[y]; });
+            for (const int i : order) {
+                if (t_idx.empty() || t_idx.back() != elem_idx[i]) {
+                    t_idx.push_back(elem_idx[i]);
+                    t_w.push_back(0.0);
+                }
+                t_w.back() += weights[i];
+            }
         }
+        const int* idx = ascending ? elem_idx : t_idx.data();
+        const double* w = ascending ? weights : t_w.data();
+        const int n_target = ascending ? n_elem : static_cast<int>(t_idx.size());
         auto a = std::make_unique<cunibs_adm>();
         a->ctx = c;
         a->dirs.n = n_dir;
@@ -1337,10 +1348,14 @@ int cunibs_adm_create(cunibs_context* c, const int* elem_idx, const double* weig
         cudaStream_t s = c->stream;
         DevArray<int> d_idx;
         DevArray<double> d_w;
-        d_idx.upload(t_idx.data(), t_idx.size(), s);
-        d_w.upload(t_w.data(), t_w.size(), s);
-        a->alpha.resize(m.n_tets);
-        adm_scatter_weights(d_idx.get(), d_w.get(), static_cast<int>(t_idx.size()), a->alpha, s);
+        if (n_target == m.n_tets) {  // every element, in order
+            a->alpha.upload(w, n_target, s);
+        } else {
+            d_idx.upload(idx, n_target, s);
+            d_w.upload(w, n_target, s);
+            a->alpha.resize(m.n_tets);
+            adm_scatter_weights(d_idx.get(), d_w.get(), n_target, a->alpha, s);
+        }
         const int K = n_dir == 1 ? 1 : (n_dir == 2 ? 2 : 4);
         const int n_red = m.n_nodes - 1;
         DevArray<double> B(static_cast<std::size_t>(n_red) * K), X(static_cast<std::size_t>(n_red) * K);

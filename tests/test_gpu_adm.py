@@ -11,6 +11,8 @@ the forward solve or the layer below it, on a multi-tissue sphere.
 
 from __future__ import annotations
 
+import time
+
 import numpy as np
 import pytest
 
@@ -186,3 +188,34 @@ def test_coverage_grid_holds_the_coil_at_every_rotation(setup):
         handles = centers + 50.0 * (np.cos(a) * v + np.sin(a) * u)
         e = adm.evaluate(recip, coil, [Placement(c, hd, DIST) for c, hd in zip(centers, handles)], DIDT)
         assert np.isfinite(e).all()
+
+
+def test_target_of_many_elements(setup):
+    """Weights of elements named out of order or twice add up; a target of every element costs no more than its upload."""
+    subj, *_ = setup
+    n = subj.context.n_tets
+    rng = np.random.default_rng(3)
+    alpha = rng.uniform(0.5, 1.5, n) / n
+
+    def solve(idx, w, tolerance=1e-9):
+        target = adm.ResolvedTarget(elem_idx=np.asarray(idx, np.int32), weights=np.asarray(w), magnitude=False,
+                                    directions=np.array([[0.0, 1.0, 0.0]]), barycenter_mm=np.zeros(3))
+        return adm.solve_adjoint(subj, target, tolerance=tolerance)
+
+    for count in (n, n // 3):
+        whole = solve(np.arange(count), alpha[:count]).node_weights
+        order = rng.permutation(count)
+        np.testing.assert_array_equal(solve(order, alpha[order]).node_weights, whole)
+        twice = np.concatenate([order, order[::2]])
+        halved = np.where(np.isin(np.arange(count), order[::2]), 0.5, 1.0) * alpha[:count]  # exact halves
+        np.testing.assert_array_equal(solve(twice, halved[twice]).node_weights, whole)
+
+    def seconds(count):
+        idx, w, times = np.arange(count), alpha[:count], []
+        for _ in range(7):
+            t = time.perf_counter()
+            solve(idx, w, 0.5).handle.close()
+            times.append(time.perf_counter() - t)
+        return np.median(times)
+
+    assert seconds(n) < seconds(10) + 50e-9 * n  # an ordered map of the elements took about 140 ns each
