@@ -7,6 +7,7 @@ be loaded, every entry point raises.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 import weakref
 from pathlib import Path
 
@@ -265,6 +266,7 @@ class Context:
         self._submitted: dict[int, tuple] = {}
         self._study: tuple | None = None
         self._adms: weakref.WeakSet = weakref.WeakSet()
+        self._selecting = threading.Lock()
         self.params = prm
         info = Info()
         check(lib.cunibs_context_info(h, C.byref(info)))
@@ -345,11 +347,12 @@ class Context:
         empty when the mesh has no element of the tissue."""
         p = np.ascontiguousarray(position_mm, np.float64).reshape(3)
         n = C.c_int(0)
-        check(self._lib.cunibs_context_select(self.handle, int(tag), _p(p), float(radius_mm), C.byref(n)))
-        idx = np.empty(n.value, np.int32)
-        rec = np.empty((n.value, 4))
-        if n.value:
-            check(self._lib.cunibs_context_selected(self.handle, _p(idx), _p(rec), n.value))
+        with self._selecting:  # the context keeps the selection from the first call to the second
+            check(self._lib.cunibs_context_select(self.handle, int(tag), _p(p), float(radius_mm), C.byref(n)))
+            idx = np.empty(n.value, np.int32)
+            rec = np.empty((n.value, 4))
+            if n.value:
+                check(self._lib.cunibs_context_selected(self.handle, _p(idx), _p(rec), n.value))
         return idx, np.ascontiguousarray(rec[:, :3]), np.ascontiguousarray(rec[:, 3])
 
     def dadt(self, coil, transforms, didt) -> np.ndarray:

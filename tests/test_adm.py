@@ -6,10 +6,14 @@ the optimiser against forward solves and a brute-force sweep) is tests/test_gpu_
 
 from __future__ import annotations
 
+import ctypes
+import threading
+import time
+
 import numpy as np
 import pytest
 
-from cunibs_b200 import adm
+from cunibs_b200 import _native, adm
 
 
 def test_target_direction_is_normalised_and_copied():
@@ -80,3 +84,49 @@ def test_exact_functional_is_the_weighted_sum():
 def test_optimize_placement_rejects_even_n_samples():
     with pytest.raises(ValueError, match="odd"):
         adm.optimize_placement(None, None, np.zeros((1, 3)), n_samples=8)
+
+
+class _Selections:
+    """A library that keeps the last selection in its context, as the native one does: of tag t, t elements t."""
+
+    def __init__(self):
+        self.tag = 0
+
+    def __getattr__(self, name):
+        return lambda *args: 0
+
+    def cunibs_context_create(self, *args):
+        args[-1]._obj.value = 1
+        return 0
+
+    def cunibs_context_select(self, handle, tag, position, radius, count):
+        self.tag = tag
+        time.sleep(1e-3)
+        count._obj.value = self.tag
+        time.sleep(1e-3)
+        return 0
+
+    def cunibs_context_selected(self, handle, idx, rec, cap):
+        n = self.tag if self.tag <= cap else cap
+        ctypes.memmove(idx, np.full(n, self.tag, np.int32).ctypes.data, 4 * n)
+        ctypes.memmove(rec, np.full(4 * n, float(self.tag)).ctypes.data, 32 * n)
+        return 0
+
+
+def test_two_threads_select_each_its_own_elements(monkeypatch):
+    monkeypatch.setattr(_native, "load", _Selections)
+    ctx = _native.Context(np.zeros((4, 3)), np.zeros((1, 4)), np.zeros(1), np.zeros((0, 3)), _native.Params())
+    wrong = []
+
+    def select(tag):
+        for _ in range(20):
+            idx, bary, vols = ctx.select_elements(tag, np.zeros(3), 1.0)
+            if not (idx.size == tag and (idx == tag).all() and (bary == tag).all() and (vols == tag).all()):
+                wrong.append((tag, idx))
+
+    threads = [threading.Thread(target=select, args=(tag,)) for tag in (2, 7)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
