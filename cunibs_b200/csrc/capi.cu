@@ -554,7 +554,7 @@ PendingBlock finish_block(cunibs_context* c, long long ticket, SolveStats& st, b
         }
         c->e_slots.reserve(static_cast<std::size_t>(op->n_slots) * 3 * k);
         apply_recovery(m, *op, c->X.get(), K, sl.dadt_nodes.get(), e_elem, k, c->e_slots.get(),
-                       want_E ? c->E.get() : nullptr, c->magn.get(), s);
+                       want_E ? c->E.get() : nullptr, c->magn.get(), c->sm_count, s);
     }
     c->summary.reserve(static_cast<std::size_t>(kSummaryLen) * k);
     gm_summary(m, c->magn.get(), k, c->summary.get(), c->sw, s);
@@ -1715,7 +1715,8 @@ int cunibs_context_recover(cunibs_context* c, int mode, int k, const double* v, 
             require(E_elem != nullptr, "SPR recovery reads E_elem");
             ee.upload(E_elem, static_cast<std::size_t>(m.n_tets) * 3 * k, s);
         }
-        apply_recovery(m, op, x.get(), k, da.get(), ee.get(), k, slots.get(), E ? Ed.get() : nullptr, mag.get(), s);
+        apply_recovery(m, op, x.get(), k, da.get(), ee.get(), k, slots.get(), E ? Ed.get() : nullptr, mag.get(),
+                       c->sm_count, s);
         copy_out(E_slots, slots.get(), sizeof(float) * slots.size(), cudaMemcpyDeviceToHost, s);
         copy_out(magnE, mag.get(), sizeof(float) * mag.size(), cudaMemcpyDeviceToHost, s);
         if (E) copy_out(E, Ed.get(), sizeof(float) * Ed.size(), cudaMemcpyDeviceToHost, s);

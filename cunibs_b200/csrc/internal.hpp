@@ -395,7 +395,7 @@ const int* recovery_slot_of_corner(const Mesh& m, const RecoveryOp& op);
 // Recovered E on slots (k, n_slots, 3) and at the barycentres: E (k,M,3) or null, magn (k,M).
 // Harmonic reads the solver block x_red (N-1, K) and dadt_nodes (k,N,3); SPR reads e_elem (k,M,3).
 void apply_recovery(const Mesh& m, const RecoveryOp& op, const double* x_red, int K, const float* dadt_nodes,
-                    const float* e_elem, int k, float* e_slots, float* E, float* magn, cudaStream_t s);
+                    const float* e_elem, int k, float* e_slots, float* E, float* magn, int sm_count, cudaStream_t s);
 
 // Conductivity Monte Carlo (sigma.cu): per-draw operator values and the sensitivity-subspace guess.
 constexpr int kSigmaMaxTags = 10;

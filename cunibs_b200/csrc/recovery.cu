@@ -540,9 +540,10 @@ __global__ void __launch_bounds__(32 * kFitWarps) harmonic_weights_kernel(const 
     if (lane == 0) status[s] = rung;
 }
 
-// The harmonic apply's entries in flight: eight where the GPU holds every thread (148 SMs of 2048), so that
-// registers cost nothing (one placement on 121k nodes: the apply 53 us at one entry); two where they queue.
-constexpr std::int64_t kFewThreads = 148 * 2048;
+// The harmonic apply's entries in flight: eight where threads are few, two where they are many and registers cost resident
+// ones. The recovery and summary of a block, eight against two: 19k threads 90 and 96 us, 165k 139 and 144, 330k 178 and
+// 178, 592k 249 and 238, 1.8M 595 and 552; the line is at 2048 threads an SM (303k on 148).
+constexpr std::int64_t kFewThreadsPerSm = 2048;
 constexpr int kEntriesFew = 8;
 constexpr int kEntriesMany = 2;
 
@@ -824,7 +825,7 @@ const int* recovery_slot_of_corner(const Mesh& m, const RecoveryOp& op) {
 }
 
 void apply_recovery(const Mesh& m, const RecoveryOp& op, const double* x_red, int K, const float* dadt_nodes,
-                    const float* e_elem, int k, float* e_slots, float* E, float* magn, cudaStream_t s) {
+                    const float* e_elem, int k, float* e_slots, float* E, float* magn, int sm_count, cudaStream_t s) {
     if (op.mode == kRecHarmonic) {
         const char* lanes = std::getenv("CUNIBS_LANE_COLUMNS");
         const int C = K % 2 == 0 && !(lanes != nullptr && lanes[0] == '1') ? 2 : 1;
@@ -835,7 +836,7 @@ void apply_recovery(const Mesh& m, const RecoveryOp& op, const double* x_red, in
                 k, e_slots);
         };
         auto pick = [&](auto cc) {
-            if (n < kFewThreads) go(cc, std::integral_constant<int, kEntriesFew>{});
+            if (n < kFewThreadsPerSm * sm_count) go(cc, std::integral_constant<int, kEntriesFew>{});
             else go(cc, std::integral_constant<int, kEntriesMany>{});
         };
         if (C == 2) pick(std::integral_constant<int, 2>{});
