@@ -271,7 +271,7 @@ void dadt_near_general(const Mesh& m, const float* dip_packed, int n_dip, const 
 
 // Records the calling thread's message for cunibs_last_error.
 void set_last_error(const std::string& message);
-// neg_vc: the per-element weights -(vol * sigma) in FP32 (null: the mesh's own).
+// The right-hand sides of the element dA/dt under the mesh's own conductivities.
 void rhs_block(const Mesh& m, const float* dadt_elm, int k, int k_pad, double* b_red /* (N-1, k_pad) */,
                cudaStream_t s);
 // The right-hand sides of n_tables (1..11) conductivity tables (n_tables, 11) in one pass: b_red (n_tables, N-1, k_pad).

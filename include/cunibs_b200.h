@@ -305,9 +305,9 @@ int cunibs_adm_destroy(cunibs_adm* adm);
 int cunibs_adm_node_weights(const cunibs_adm* adm, double* out);
 
 /* Samples Q_d(g) = mu0/4pi sum_n W_d[n] x (g - r_n) / |g - r_n|^3 on a regular grid (origin and
- * spacing in mm, shape per axis; C order, x slowest) with the FP32 dipole N-body centred on the
- * grid's centre (replaces sample_qfield, reciprocity.py:183-213). The field stays on the device, complete when
- * the call returns. */
+ * spacing in mm, shape per axis; C order, x slowest) in FP32 (replaces sample_qfield, reciprocity.py:183-213): about the
+ * centre c of a tile of points, two sums over the nodes, (sum w W) x (g - c) - sum w (W x (r - c)), and the cross products
+ * themselves for nodes near the tile. The field stays on the device, complete when the call returns. */
 int cunibs_adm_sample(cunibs_adm* adm, const double* origin_mm, const double* spacing_mm, const int* shape);
 
 /* Copies the sampled field (n_dir, nx, ny, nz, 3) FP32 to host memory (cap: floats available). */

@@ -10,6 +10,7 @@ rounding: 16 u |W| / |g - r|^2.
 
 from __future__ import annotations
 
+import dataclasses
 import time
 
 import numpy as np
@@ -26,8 +27,9 @@ pytestmark = pytest.mark.gpu
 def adjoints(request):
     subj = Subject(sphere_head(request.param, 90.0, jitter_mm=0.2, seed=4), tolerance=1e-9)
     focus = [3.0, 2.0, 60.0]
-    yield [adm.solve_adjoint(subj, adm.resolve_target(subj, adm.Target(focus, d, radius_mm=20.0)))
-           for d in ((0.0, 1.0, 0.0), None)]
+    found = [adm.resolve_target(subj, adm.Target(focus, d, radius_mm=20.0)) for d in ((0.0, 1.0, 0.0), None)]
+    found.append(dataclasses.replace(found[1], directions=np.eye(3)[:2]))  # two directions
+    yield [adm.solve_adjoint(subj, target) for target in found]
     subj.free()
 
 
